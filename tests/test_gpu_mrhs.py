@@ -114,3 +114,23 @@ def test_multi_rhs_timing_entry_points(q, fields):
     x = dev(np.zeros((4,) + tuple(O.full_shape(f["latt"])), dtype=np.complex128))
     ms2, tune = q.batch_dslash_time([(f["G"], x, b, 0.12, False)], precision=32, gauge_precision=16, iters=3)
     assert 0.0 < ms2 < 1e3 and tune["dslash_threads"] in (32, 64, 128, 256)
+
+
+@pytest.mark.parametrize("latt", [[2, 3, 3, 4], [6, 3, 1, 5]])
+@pytest.mark.parametrize("nrhs", [12, 65])
+def test_multi_rhs_ragged_site_tiles(q, latt, nrhs):
+    """Site counts (36, 45) that end inside a tile of the layout kernels (8 sites up to 64 rows, 4 above); one site
+    past the output's end stays as it was."""
+    import torch
+
+    U = O.gauge_smooth(latt, 0.25, 75)
+    psi = np.stack([O.fermion_gauss(O.half_shape(latt), 950 + j) for j in range(nrhs)])
+    inp = dev(psi)
+    buf = torch.full((inp.numel() + 12,), float("nan"), dtype=inp.dtype, device=inp.device)
+    out = buf[:inp.numel()].view(inp.shape)
+    with q.Gauge(dev(U), latt) as G:
+        for par in (0, 1):
+            G.dslash_multi_tc(out, inp, nrhs, par)
+            got = host(out)
+            assert max(rel(got[j], O.dslash(psi[j], U, latt, par, 1.0)) for j in range(nrhs)) < BAR
+    assert bool(torch.isnan(buf[inp.numel():].real).all())

@@ -21,240 +21,361 @@ namespace qcu {
 
 using C = Cpx<double>;
 
-__device__ __forceinline__ void m3_mul(const C *a, const C *b, C *c) {
-  C t[9];
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int k = 0; k < 3; k++) t[r * 3 + k] = a[r * 3] * b[k] + a[r * 3 + 1] * b[3 + k] + a[r * 3 + 2] * b[6 + k];
-#pragma unroll
-  for (int i = 0; i < 9; i++) c[i] = t[i];
+// acc += a b, acc += conj(a) b: four fused multiply-adds each
+__device__ __forceinline__ void cmad(C &acc, const C &a, const C &b) {
+  acc.re = fma(-a.im, b.im, fma(a.re, b.re, acc.re));
+  acc.im = fma(a.im, b.re, fma(a.re, b.im, acc.im));
 }
-__device__ __forceinline__ void m3_dag(C *a) {
-  C t[9];
-#pragma unroll
-  for (int r = 0; r < 3; r++)
-#pragma unroll
-    for (int k = 0; k < 3; k++) t[r * 3 + k] = a[k * 3 + r].conj();
-#pragma unroll
-  for (int i = 0; i < 9; i++) a[i] = t[i];
+__device__ __forceinline__ void cmadc(C &acc, const C &a, const C &b) {
+  acc.re = fma(a.im, b.im, fma(a.re, b.re, acc.re));
+  acc.im = fma(-a.im, b.re, fma(a.re, b.im, acc.im));
 }
 
-// link U_mu at full coordinate (x,y,z,t) (wrapped), from the PyQuda gauge
-__device__ __forceinline__ void link_at(const GaugeView<GAOS64> &U, const Geom &g, int x, int y, int z, int t, int mu,
-                                        C *u) {
-  const int Lx = 2 * g.Lxh;
-  x = (x + Lx) % Lx;
-  y = (y + g.Ly) % g.Ly;
-  z = (z + g.Lz) % g.Lz;
-  t = (t + g.Lt) % g.Lt;
-  const int par = (x + y + z + t) & 1;
-  const int s = ((t * g.Lz + z) * g.Ly + y) * g.Lxh + (x >> 1);
-  link_load<GAOS64, double>(U, mu, par, s, u);
-}
-
-// sum of the four leaves in plane (mu, nu) at c[] (same products as qcu, in the
-// same left-to-right order)
-__device__ __noinline__ void clover_leaves(const GaugeView<GAOS64> &U, const Geom &g, const int c[4], int mu, int nu,
-                                           C *Q) {
-  int a[4], b[4];
-  C u1[9], u2[9], u3[9], u4[9], t[9];
-#define SH(dst, src, d, st)                 \
-  {                                         \
-    for (int q = 0; q < 4; q++) dst[q] = src[q]; \
-    dst[d] += st;                           \
-  }
-#define LK(p, d, u) link_at(U, g, p[0], p[1], p[2], p[3], d, u)
+// a <- a b and a <- a b^dag, row by row in place
+__device__ __forceinline__ void mul_nn(C *a, const C *b) {
 #pragma unroll
-  for (int k = 0; k < 9; k++) Q[k] = C(0, 0);
-  // U_mu(x) U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+
-  LK(c, mu, u1);
-  SH(a, c, mu, 1);
-  LK(a, nu, u2);
-  SH(a, c, nu, 1);
-  LK(a, mu, u3);
-  LK(c, nu, u4);
-  m3_mul(u1, u2, t);
-  m3_dag(u3);
-  m3_mul(t, u3, t);
-  m3_dag(u4);
-  m3_mul(t, u4, t);
+  for (int r = 0; r < 3; r++) {
+    const C u = a[r * 3], v = a[r * 3 + 1], w = a[r * 3 + 2];
 #pragma unroll
-  for (int k = 0; k < 9; k++) Q[k] += t[k];
-  // U_nu(x) U_mu(x-mu+nu)^+ U_nu(x-mu)^+ U_mu(x-mu)
-  LK(c, nu, u1);
-  SH(a, c, mu, -1);
-  SH(b, a, nu, 1);
-  LK(b, mu, u2);
-  LK(a, nu, u3);
-  LK(a, mu, u4);
-  m3_dag(u2);
-  m3_mul(u1, u2, t);
-  m3_dag(u3);
-  m3_mul(t, u3, t);
-  m3_mul(t, u4, t);
-#pragma unroll
-  for (int k = 0; k < 9; k++) Q[k] += t[k];
-  // U_mu(x-mu)^+ U_nu(x-mu-nu)^+ U_mu(x-mu-nu) U_nu(x-nu)
-  SH(a, c, mu, -1);
-  LK(a, mu, u1);
-  SH(b, a, nu, -1);
-  LK(b, nu, u2);
-  LK(b, mu, u3);
-  SH(a, c, nu, -1);
-  LK(a, nu, u4);
-  m3_dag(u1);
-  m3_dag(u2);
-  m3_mul(u1, u2, t);
-  m3_mul(t, u3, t);
-  m3_mul(t, u4, t);
-#pragma unroll
-  for (int k = 0; k < 9; k++) Q[k] += t[k];
-  // U_nu(x-nu)^+ U_mu(x-nu) U_nu(x+mu-nu) U_mu(x)^+
-  SH(a, c, nu, -1);
-  LK(a, nu, u1);
-  LK(a, mu, u2);
-  SH(b, a, mu, 1);
-  LK(b, nu, u3);
-  LK(c, mu, u4);
-  m3_dag(u1);
-  m3_mul(u1, u2, t);
-  m3_mul(t, u3, t);
-  m3_dag(u4);
-  m3_mul(t, u4, t);
-#pragma unroll
-  for (int k = 0; k < 9; k++) Q[k] += t[k];
-#undef SH
-#undef LK
-}
-
-__device__ __forceinline__ C unit(int re, int im) { return C((double)re, (double)im); }
-
-// packed block store (site-blocked CSOA64): d[0..5] then lower triangle
-__device__ __forceinline__ void block_store(void *out, int blk, int s, const C M[36]) {
-  double2 *p = static_cast<double2 *>(out) + blk_base<36>(s) + blk * 18 * SB;
-  p[0] = make_double2(M[0].re, M[7].re);
-  p[SB] = make_double2(M[14].re, M[21].re);
-  p[2 * SB] = make_double2(M[28].re, M[35].re);
-  int k = 3;
-  for (int i = 1; i < 6; i++)
-    for (int j = 0; j < i; j++, k++) p[k * SB] = make_double2(M[i * 6 + j].re, M[i * 6 + j].im);
-}
-
-// Hermitian inverse of a 6x6 block by LDL^H; returns false on a zero pivot
-__device__ bool herm6_inverse(const C A[36], C Ai[36]) {
-  C L[36];
-  double D[6];
-#pragma unroll
-  for (int j = 0; j < 6; j++) {
-    double dj = A[j * 6 + j].re;
-#pragma unroll
-    for (int k = 0; k < j; k++) dj -= L[j * 6 + k].norm2() * D[k];
-    if (dj == 0.0 || !(dj == dj)) return false;
-    D[j] = dj;
-#pragma unroll
-    for (int i = j + 1; i < 6; i++) {
-      C v = A[i * 6 + j];
-#pragma unroll
-      for (int k = 0; k < j; k++) v -= L[i * 6 + k] * L[j * 6 + k].conj() * D[k];
-      L[i * 6 + j] = v * (1.0 / dj);
+    for (int k = 0; k < 3; k++) {
+      C t = u * b[k];
+      cmad(t, v, b[3 + k]);
+      cmad(t, w, b[6 + k]);
+      a[r * 3 + k] = t;
     }
   }
-  // M = L^-1 (unit lower triangular)
-  C M[36];
+}
+__device__ __forceinline__ void mul_nd(C *a, const C *b) {
 #pragma unroll
-  for (int j = 0; j < 6; j++) {
+  for (int r = 0; r < 3; r++) {
+    const C u = a[r * 3], v = a[r * 3 + 1], w = a[r * 3 + 2];
 #pragma unroll
-    for (int i = 0; i < 6; i++) M[i * 6 + j] = C(i == j ? 1.0 : 0.0, 0.0);
-#pragma unroll
-    for (int i = j + 1; i < 6; i++) {
-      C v(0, 0);
-#pragma unroll
-      for (int k = j; k < i; k++) v += L[i * 6 + k] * M[k * 6 + j];
-      M[i * 6 + j] = -v;
+    for (int k = 0; k < 3; k++) {
+      C t = cdotmul(b[k * 3], u);
+      cmadc(t, b[k * 3 + 1], v);
+      cmadc(t, b[k * 3 + 2], w);
+      a[r * 3 + k] = t;
     }
   }
-  // A^-1 = M^H D^-1 M
+}
+// d -= a^dag b
+__device__ __forceinline__ void sub_dn(C *d, const C *a, const C *b) {
 #pragma unroll
-  for (int i = 0; i < 6; i++)
+  for (int c = 0; c < 3; c++)
 #pragma unroll
-    for (int j = 0; j <= i; j++) {
-      C v(0, 0);
+    for (int r = 0; r < 3; r++) {
+      const C m(-a[c * 3 + r].re, -a[c * 3 + r].im);
 #pragma unroll
-      for (int k = i; k < 6; k++) v += M[k * 6 + i].conj() * M[k * 6 + j] * (1.0 / D[k]);
-      Ai[i * 6 + j] = v;
-      Ai[j * 6 + i] = v.conj();
+      for (int k = 0; k < 3; k++) cmadc(d[r * 3 + k], m, b[c * 3 + k]);
     }
-  return true;
+}
+// f += w - w^dag: the imaginary parts of the diagonal, then the entries (1,0), (2,0), (2,1)
+__device__ __forceinline__ void add_antiherm(double f[9], const C *w) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) f[k] += 2.0 * w[4 * k].im;
+  f[3] += w[3].re - w[1].re;
+  f[4] += w[3].im + w[1].im;
+  f[5] += w[6].re - w[2].re;
+  f[6] += w[6].im + w[2].im;
+  f[7] += w[7].re - w[5].re;
+  f[8] += w[7].im + w[5].im;
 }
 
-__global__ void k_clover_build(Geom g, GaugeView<GAOS64> U, int par, double coeff, void *A64, void *Ainv64,
-                               int *bad) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.Vh) return;
-  const int xh = s % g.Lxh;
-  int r = s / g.Lxh;
-  const int y = r % g.Ly;
-  r /= g.Ly;
-  const int z = r % g.Lz;
-  const int t = r / g.Lz;
-  const int c[4] = {2 * xh + ((y + z + t + par) & 1), y, z, t};
-  // every loop below is unrolled, so blk is indexed at compile time and
-  // stays in registers (a runtime index would place it in local memory)
-  C blk[2][36];
+// a site by its full coordinates, and its neighbour one step (st = +1 or -1) along d, periodic
+struct Pos {
+  int x, y, z, t;
+};
+__device__ __forceinline__ int wrap_step(int v, int L, int st) {
+  v += st;
+  return v == L ? 0 : (v < 0 ? L - 1 : v);
+}
+__device__ __forceinline__ Pos step(const Geom &g, Pos c, int d, int st) {
+  if (d == 0) c.x = wrap_step(c.x, 2 * g.Lxh, st);
+  else if (d == 1) c.y = wrap_step(c.y, g.Ly, st);
+  else if (d == 2) c.z = wrap_step(c.z, g.Lz, st);
+  else c.t = wrap_step(c.t, g.Lt, st);
+  return c;
+}
+
+// Links staged ahead of their use: every thread copies the rows 0 and 1 of its
+// own links into its own slots of shared memory (cp.async, 16 bytes a lane and
+// row element, so a warp's accesses are contiguous) and reads them back when
+// their turn comes, two links later: no barrier, and no registers held by
+// loads in flight.
+constexpr int CL_SLOTS = 3;
+constexpr int CL_SLOT_BYTES = 6 * 16 * 32;  // one warp's links
+template <int G>
+struct LinkStage {
+  GaugeView<G> U;
+  Geom g;
+  unsigned slot0;  // this lane's 16 bytes of element 0 of slot 0
+  const double2 *slot0p;
+  __device__ __forceinline__ void fetch(int i, const Pos &c, int mu) const {
+    const int s = ((c.t * g.Lz + c.z) * g.Ly + c.y) * g.Lxh + (c.x >> 1);
+    const size_t slab = (size_t)(mu * 2 + ((c.x + c.y + c.z + c.t) & 1)) * U.stride;
+    const double2 *p = static_cast<const double2 *>(U.p) + (G == GAOS64 ? (slab + s) * 9 : slab * 6 + blk_base<6>(s));
+    const unsigned d = slot0 + (i % CL_SLOTS) * CL_SLOT_BYTES;
 #pragma unroll
-  for (int b = 0; b < 2; b++)
+    for (int k = 0; k < 6; k++)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + k * 512), "l"(p + (G == GAOS64 ? k : k * SB))
+                   : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // link i, once at most `pending` later fetches are still in flight
+  template <int PENDING>
+  __device__ __forceinline__ void take(int i, C *m) const {
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+    const double2 *p = slot0p + (i % CL_SLOTS) * (CL_SLOT_BYTES / 16);
 #pragma unroll
-    for (int k = 0; k < 36; k++) blk[b][k] = C(0, 0);
+    for (int k = 0; k < 6; k++) {
+      const double2 v = p[k * 32];
+      m[k] = C(v.x, v.y);
+    }
+    m[6] = row2(m[1], m[5], m[2], m[4]);
+    m[7] = row2(m[2], m[3], m[0], m[5]);
+    m[8] = row2(m[0], m[4], m[1], m[3]);
+  }
+  // conj(a b - c d), the cross product's component, in fused multiply-adds
+  static __device__ __forceinline__ C row2(const C &a, const C &b, const C &c, const C &d) {
+    C v = a * b;
+    cmad(v, C(-c.re, -c.im), d);
+    return v.conj();
+  }
+};
+
+// Q - Q^dag of the plane (mu, nu) at c, Q the sum of the four plaquette
+// leaves.  Two leaves begin with U_mu(x), two end with U_mu(x - mu), and a leaf
+// may be replaced by minus its adjoint, so
+//   W = U_mu(x) (S1 - S2) + (S3 - S4) U_mu(x - mu),   Q - Q^dag = W - W^dag
+// with the staples
+//   S1 = U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+         S3 = U_nu(x) U_mu(x-mu+nu)^+ U_nu(x-mu)^+
+//   S2 = (U_mu(x-nu) U_nu(x+mu-nu))^+ U_nu(x-nu)   S4 = (U_mu(x-mu-nu) U_nu(x-nu))^+ U_nu(x-mu-nu)
+// : ten 3x3 products a plane where the leaves one by one take twelve.
+// The products run in place (three matrices live at a time).
+template <int G>
+__device__ __forceinline__ void clover_plane(const LinkStage<G> &S, const Pos &c, int mu, int nu, double f[9]) {
+  const Geom &g = S.g;
+  C a[9], b[9], d[9];
+#pragma unroll
+  for (int k = 0; k < 9; k++) f[k] = 0.0;
+  const Pos xm = step(g, c, mu, -1), xn = step(g, c, nu, -1), xmn = step(g, xm, nu, -1);
+  S.fetch(0, step(g, c, mu, 1), nu);
+  S.fetch(1, step(g, c, nu, 1), mu);
+  S.fetch(2, c, nu);
+  S.template take<2>(0, d);
+  S.template take<1>(1, b);
+  mul_nd(d, b);
+  S.fetch(3, xn, mu);
+  S.fetch(4, step(g, xn, mu, 1), nu);
+  S.template take<2>(2, b);
+  mul_nd(d, b);
+  S.fetch(5, xn, nu);
+  S.template take<2>(3, a);
+  S.template take<1>(4, b);
+  mul_nn(a, b);
+  S.fetch(6, c, mu);
+  S.fetch(7, c, nu);
+  S.template take<2>(5, b);
+  sub_dn(d, a, b);
+  S.fetch(8, step(g, xm, nu, 1), mu);
+  S.template take<2>(6, a);
+  mul_nn(a, d);
+  add_antiherm(f, a);
+  S.fetch(9, xm, nu);
+  S.template take<2>(7, d);
+  S.template take<1>(8, b);
+  mul_nd(d, b);
+  S.fetch(10, xmn, mu);
+  S.fetch(11, xn, nu);
+  S.template take<2>(9, b);
+  mul_nd(d, b);
+  S.fetch(12, xmn, nu);
+  S.template take<2>(10, a);
+  S.template take<1>(11, b);
+  mul_nn(a, b);
+  S.fetch(13, xm, mu);
+  S.template take<1>(12, b);
+  sub_dn(d, a, b);
+  S.template take<0>(13, a);
+  mul_nn(d, a);
+  add_antiherm(f, d);
+}
+
+// packed lower triangle of a Hermitian 6x6 block: diagonal d, (i, j), i > j, at tri(i, j)
+__host__ __device__ constexpr int tri(int i, int j) { return i * (i - 1) / 2 + j; }
+
+// Chiral block B (spins 2B, 2B+1) of A = 1 + scale sum_{mu<nu} gamma_mu
+// gamma_nu F_munu from the six planes' F of one site (F[9 * plane + e] at
+// stride SB); only the lower triangle is formed.
+template <int B>
+__device__ __forceinline__ void clover_block(const double *F, double scale, double d[6], C L[15]) {
+#pragma unroll
+  for (int k = 0; k < 6; k++) d[k] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 15; k++) L[k] = C(0, 0);
+  int plane = 0;
 #pragma unroll
   for (int mu = 0; mu < 4; mu++)
 #pragma unroll
-    for (int nu = mu + 1; nu < 4; nu++) {
-      C Q[9], F[9];
-      clover_leaves(U, g, c, mu, nu, Q);
+    for (int nu = mu + 1; nu < 4; nu++, plane++) {
+      double f[9];
 #pragma unroll
-      for (int i = 0; i < 3; i++)
+      for (int e = 0; e < 9; e++) f[e] = F[(plane * 9 + e) * SB];
 #pragma unroll
-        for (int k = 0; k < 3; k++) F[i * 3 + k] = Q[i * 3 + k] - Q[k * 3 + i].conj();
-#pragma unroll
-      for (int s0 = 0; s0 < 4; s0++) {
+      for (int h = 0; h < 2; h++) {
+        const int s0 = 2 * B + h;
         const int j = gcol(mu, s0), s1 = gcol(nu, j);
-        const C sv = unit(gre(mu, s0), gim(mu, s0)) * unit(gre(nu, j), gim(nu, j));
-        const int b = s0 >> 1, r0 = (s0 & 1) * 3, c0 = (s1 & 1) * 3;
+        const int vr = gre(mu, s0) * gre(nu, j) - gim(mu, s0) * gim(nu, j);
+        const int vi = gre(mu, s0) * gim(nu, j) + gim(mu, s0) * gre(nu, j);
+        const int r0 = h * 3, c0 = (s1 & 1) * 3;
 #pragma unroll
         for (int i = 0; i < 3; i++)
 #pragma unroll
-          for (int k = 0; k < 3; k++) blk[b][(r0 + i) * 6 + c0 + k] += sv * F[i * 3 + k];
+          for (int k = 0; k < 3; k++) {
+            if (r0 + i < c0 + k) continue;
+            const int e = i > k ? 3 + 2 * tri(i, k) : 3 + 2 * tri(k, i);
+            const C v = i == k ? C(0.0, f[i]) : (i > k ? C(f[e], f[e + 1]) : C(-f[e], f[e + 1]));
+            // times vr + i vi, one of 1, -1, i, -i (known when unrolled)
+            const C u = vr == 1 ? v : (vr == -1 ? -v : (vi == 1 ? C(-v.im, v.re) : C(v.im, -v.re)));
+            if (r0 + i == c0 + k) d[r0 + i] += u.re;
+            else L[tri(r0 + i, c0 + k)] += u;
+          }
       }
     }
 #pragma unroll
-  for (int b = 0; b < 2; b++) {
+  for (int k = 0; k < 6; k++) d[k] = 1.0 + d[k] * scale;
 #pragma unroll
-    for (int k = 0; k < 36; k++) blk[b][k] = blk[b][k] * (-0.125 * coeff);
+  for (int k = 0; k < 15; k++) L[k] = L[k] * scale;
+}
+
+// In place: the block A (d, L) -> M = L^-1 of A = L D L^H and 1 / D, so that
+// A^-1 = M^H D^-1 M.  False on a zero or undefined pivot.
+__device__ __forceinline__ bool ldl6(double d[6], C L[15]) {
+  bool ok = true;
 #pragma unroll
-    for (int k = 0; k < 6; k++) blk[b][k * 7] += C(1.0, 0.0);
-    if (A64) block_store(A64, b, s, blk[b]);
-    if (Ainv64) {
-      C inv[36];
-      if (!herm6_inverse(blk[b], inv)) {
-        atomicAdd(bad, 1);
-        for (int k = 0; k < 36; k++) inv[k] = C(0, 0);
-      }
-      block_store(Ainv64, b, s, inv);
+  for (int j = 0; j < 6; j++) {
+#pragma unroll
+    for (int k = 0; k < j; k++) d[j] -= L[tri(j, k)].norm2() * d[k];
+    ok = ok && d[j] != 0.0 && d[j] == d[j];
+    const double inv = 1.0 / d[j];
+#pragma unroll
+    for (int i = j + 1; i < 6; i++) {
+      C v = L[tri(i, j)];
+#pragma unroll
+      for (int k = 0; k < j; k++) v -= L[tri(i, k)] * L[tri(j, k)].conj() * d[k];
+      L[tri(i, j)] = v * inv;
     }
+  }
+  // M_ij = -(L_ij + sum_{j<k<i} L_ik M_kj): row by row, columns upwards, so
+  // that every L_ik (k > j) is read before it is overwritten
+#pragma unroll
+  for (int i = 1; i < 6; i++)
+#pragma unroll
+    for (int j = 0; j < i; j++) {
+      C v = L[tri(i, j)];
+#pragma unroll
+      for (int k = j + 1; k < i; k++) v += L[tri(i, k)] * L[tri(k, j)];
+      L[tri(i, j)] = -v;
+    }
+#pragma unroll
+  for (int k = 0; k < 6; k++) d[k] = 1.0 / d[k];
+  return ok;
+}
+
+// entry (i, j), i >= j, of M^H D^-1 M
+__device__ __forceinline__ C inv6_entry(const double d[6], const C L[15], int i, int j) {
+  C v(0, 0);
+#pragma unroll
+  for (int k = i; k < 6; k++) {
+    const C a = k == i ? C(d[k], 0.0) : L[tri(k, i)].conj() * d[k];
+    if (k == j) v += a;
+    else v += a * L[tri(k, j)];
+  }
+  return v;
+}
+
+// Writes one block in the packed form (18 double2: the diagonal in pairs, then
+// the lower triangle row by row), also as 9 float4 where o32 is given; entry(k)
+// returns double2 k.
+template <typename F>
+__device__ __forceinline__ void block_write(double2 *o64, float4 *o32, F entry) {
+#pragma unroll
+  for (int k = 0; k < 18; k += 2) {
+    const double2 u = entry(k), w = entry(k + 1);
+    o64[k * SB] = u;
+    o64[(k + 1) * SB] = w;
+    if (o32) o32[(k / 2) * SB] = make_float4((float)u.x, (float)u.y, (float)w.x, (float)w.y);
   }
 }
 
-__global__ void k_clover_to32(int Vh, const double2 *in, float4 *out) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < Vh; s += gridDim.x * blockDim.x) {
-    const double2 *pi = in + blk_base<36>(s);
-    float4 *po = out + blk_base<18>(s);
-    for (int b = 0; b < 2; b++)
-      for (int k = 0; k < 9; k++) {
-        const double2 u = pi[(b * 18 + 2 * k) * SB], w = pi[(b * 18 + 2 * k + 1) * SB];
-        po[(b * 9 + k) * SB] = make_float4((float)u.x, (float)u.y, (float)w.x, (float)w.y);
-      }
+template <int B>
+__device__ __forceinline__ void clover_finish(const double *F, double scale, int s, const CloverOut &o, int q) {
+  double d[6];
+  C L[15];
+  clover_block<B>(F, scale, d, L);
+  constexpr int row[15] = {1, 2, 2, 3, 3, 3, 4, 4, 4, 4, 5, 5, 5, 5, 5};
+  constexpr int col[15] = {0, 0, 1, 0, 1, 2, 0, 1, 2, 3, 0, 1, 2, 3, 4};
+  // selected, not indexed: a run-time index would copy the parameters to local memory
+  void *const A64 = q ? o.A64[1] : o.A64[0], *const Ainv64 = q ? o.Ainv64[1] : o.Ainv64[0],
+       *const Ainv32 = q ? o.Ainv32[1] : o.Ainv32[0];
+  if (A64)
+    block_write(static_cast<double2 *>(A64) + blk_base<36>(s) + B * 18 * SB, nullptr, [&](int k) {
+      return k < 3 ? make_double2(d[2 * k], d[2 * k + 1]) : make_double2(L[k - 3].re, L[k - 3].im);
+    });
+  if (!Ainv64) return;
+  const bool ok = ldl6(d, L);
+  if (!ok) atomicAdd(o.bad, 1);
+  float4 *o32 = Ainv32 ? static_cast<float4 *>(Ainv32) + blk_base<18>(s) + B * 9 * SB : nullptr;
+  block_write(static_cast<double2 *>(Ainv64) + blk_base<36>(s) + B * 18 * SB, o32, [&](int k) {
+    if (!ok) return make_double2(0.0, 0.0);
+    if (k < 3) return make_double2(inv6_entry(d, L, 2 * k, 2 * k).re, inv6_entry(d, L, 2 * k + 1, 2 * k + 1).re);
+    const C v = inv6_entry(d, L, row[k - 3], col[k - 3]);
+    return make_double2(v.re, v.im);
+  });
+}
+
+// The clover term and its inverse, 32 sites of one parity at a time: warp p
+// forms plane p's F for the sites (lane = site, so the loads of the
+// site-blocked links are contiguous and nothing diverges).  After `groups`
+// (1 or 3) such rounds a warp per 32 sites and chiral block assembles,
+// factorises and writes it: with three rounds all six warps have one.  Bound
+// by FP64 arithmetic (10 products and 14 link reconstructions a plane, 1.4
+// kFMA, and ~1.4 kFMA a chiral block) at the latency of its link loads; a
+// thread per site and plane keeps the working set (three 3x3 matrices and a
+// sum) in registers, where one thread for all planes held the 72-entry blocks
+// as well and its leaves went through a call with local arrays (24^3 x 48,
+// one parity: 1158 -> 341 us, FP64 pipe 58 % busy).
+constexpr int CB_THREADS = 192;
+constexpr int CB_GROUPS = 3;
+constexpr int CB_SMEM = (CB_THREADS / 32) * CL_SLOTS * CL_SLOT_BYTES + CB_GROUPS * 6 * 9 * SB * (int)sizeof(double);
+template <int G>
+__global__ void __launch_bounds__(CB_THREADS, 2) k_clover_build(Geom g, GaugeView<G> U, double scale, CloverOut o,
+                                                               int groups) {
+  extern __shared__ __align__(16) unsigned char cb_smem[];
+  double *F = reinterpret_cast<double *>(cb_smem + (CB_THREADS / 32) * CL_SLOTS * CL_SLOT_BYTES);  // [group][9 plane + e][site]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int s0 = blockIdx.x * groups * SB, q = blockIdx.y;
+  const int mu = warp < 3 ? 0 : (warp < 5 ? 1 : 2), nu = warp < 3 ? warp + 1 : (warp < 5 ? warp - 1 : 3);
+  unsigned char *slot = cb_smem + warp * CL_SLOTS * CL_SLOT_BYTES + lane * 16;
+  const LinkStage<G> S{U, g, (unsigned)__cvta_generic_to_shared(slot), reinterpret_cast<const double2 *>(slot)};
+  for (int k = 0; k < groups; k++) {
+    const int s = s0 + k * SB + lane;
+    if (s >= g.Vh) break;
+    Pos c;
+    int xh;
+    site_coords(g, s, xh, c.y, c.z, c.t);
+    c.x = 2 * xh + ((c.y + c.z + c.t + o.par0 + q) & 1);
+    double f[9];
+    clover_plane<G>(S, c, mu, nu, f);
+#pragma unroll
+    for (int e = 0; e < 9; e++) F[((k * 6 + warp) * 9 + e) * SB + lane] = f[e];
   }
+  __syncthreads();
+  const int k = warp >> 1, s = s0 + k * SB + lane;
+  if (k >= groups || s >= g.Vh) return;
+  const double *Fk = F + k * 6 * 9 * SB + lane;
+  if (warp & 1) clover_finish<1>(Fk, scale, s, o, q);
+  else clover_finish<0>(Fk, scale, s, o, q);
 }
 
 template <int K>
@@ -269,14 +390,20 @@ __global__ void k_clover_apply(int Vh, CloverView<CSOA64> cv, const void *in, vo
 
 size_t clover_bytes(int ckind, int Vh) { return (size_t)2 * (ckind == CSOA64 ? 18 * 16 : 9 * 16) * pad_sites(Vh); }
 
-void launch_clover_build(const Geom &g, const void *gauge_pyq, int par, double coeff, void *A64, void *Ainv64, int *bad,
+void launch_clover_build(int gkind, const Geom &g, const void *gauge, int nparities, double coeff, const CloverOut &o,
                          cudaStream_t s) {
-  k_clover_build<<<(g.Vh + 63) / 64, 64, 0, s>>>(g, GaugeView<GAOS64>{gauge_pyq, g.Vh}, par, coeff, A64, Ainv64, bad);
-  QCU_CHECK_LAUNCH();
-}
-
-void launch_clover_to32(int Vh, const void *c64, void *c32, cudaStream_t s) {
-  k_clover_to32<<<blas_grid(Vh), BLAS_BLOCK, 0, s>>>(Vh, static_cast<const double2 *>(c64), static_cast<float4 *>(c32));
+  // three rounds a block once that still fills every SM with its two blocks
+  // (below, the shorter blocks finish sooner than the balance of the last phase gains)
+  const int blocks = (g.Vh + SB - 1) / SB;
+  const int groups = (int64_t)blocks * nparities >= 148 * 2 * CB_GROUPS * 2 ? CB_GROUPS : 1;
+  const dim3 grid((blocks + groups - 1) / groups, nparities);
+  auto run = [&](auto kernel, auto view) {
+    QCU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CB_SMEM));
+    kernel<<<grid, CB_THREADS, CB_SMEM, s>>>(g, view, -0.125 * coeff, o, groups);
+  };
+  if (gkind == GSOA64) run(k_clover_build<GSOA64>, GaugeView<GSOA64>{gauge, pad_sites(g.Vh)});
+  else if (gkind == GAOS64) run(k_clover_build<GAOS64>, GaugeView<GAOS64>{gauge, g.Vh});
+  else throw Error(1, "clover build: unsupported gauge kind");
   QCU_CHECK_LAUNCH();
 }
 

@@ -249,6 +249,15 @@ void launch_dslash(int kind, int gkind, int ckind, const Geom &g, const DslashAr
       al32(a.x2) && al32(a.rt))
     launch_clov<AOS64W, GAOS64, CSOA64>(g, a, ctx, s);
   else if (kind == AOS64 && gkind == GAOS64 && ckind == CSOA64) launch_clov<AOS64, GAOS64, CSOA64>(g, a, ctx, s);
+  else if (kind == AOS64 && gkind == GSOA64 && ckind == CSOA64) {
+    // PyQuda-layout spinors on packed links: the hop with or without the inverse clover
+    require(a.x1 == nullptr && a.x2 == nullptr && a.red == RED_NONE, "dslash: no epilogue on this storage combination");
+    const bool wide = al32(a.in) && al32(a.out);
+    if (wide && a.clover) launch_t<AOS64W, GSOA64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
+    else if (wide) launch_t<AOS64W, GSOA64, CSOA64, false, 0, RED_NONE>(g, a, ctx, s);
+    else if (a.clover) launch_t<AOS64, GSOA64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
+    else launch_t<AOS64, GSOA64, CSOA64, false, 0, RED_NONE>(g, a, ctx, s);
+  }
   else if (kind == SOA64 && gkind == GSOA64 && ckind == CSOA64) launch_clov<SOA64, GSOA64, CSOA64>(g, a, ctx, s);
   else if (kind == SOA32 && gkind == GSOA32 && ckind == CSOA32) launch_clov<SOA32, GSOA32, CSOA32>(g, a, ctx, s);
   else if (kind == SOA16 && gkind == GSOA16 && ckind == CSOA32) launch_clov<SOA16, GSOA16, CSOA32>(g, a, ctx, s);

@@ -73,6 +73,7 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf();
   void ensure(size_t bytes);  // grow-only
+  bool try_ensure(size_t bytes);  // false (and the buffer empty) where there is no memory for it
   void release();
   template <typename T>
   T *as() const {
@@ -104,10 +105,11 @@ struct Context {
   size_t partials_blocks = 0;
   int sms = 148;                   // multiprocessors of the device
   // scratch of the legacy clover call (dslashCloverQcu): the inverse clover
-  // of the output parity and its zero-pivot counter.  Per device, used only
-  // under `mu`; allocated on first use and kept until exit.
+  // of the output parity, its zero-pivot counter and the packed links.  Per
+  // device, used only under `mu`; allocated on first use and kept until exit.
   DevBuf *legacy_clover = nullptr;
   DevBuf *legacy_bad = nullptr;
+  DevBuf *legacy_gauge = nullptr;
   std::mutex mu;
   void ensure_partials(size_t blocks);
 };
@@ -177,11 +179,17 @@ void launch_dots(int kind, int Vh, void *a, float *an, void *b, float *bn, Conte
 void launch_gauge_pack(int gkind, const Geom &g, const void *pyq, void *out, cudaStream_t s);
 size_t gauge_bytes(int gkind, int Vh);
 
-// clover: build A = 1 - coeff/8 sum g_mu g_nu (Q - Q^+) on parity `par` from the
-// PyQuda gauge, packed (CSOA64); optionally also its inverse
-void launch_clover_build(const Geom &g, const void *gauge_pyq, int par, double coeff, void *A64, void *Ainv64,
-                         int *bad, cudaStream_t s);
-void launch_clover_to32(int Vh, const void *c64, void *c32, cudaStream_t s);
+// clover: build A = 1 - coeff/8 sum g_mu g_nu (Q - Q^+) on parities par0 ..
+// par0 + nparities - 1 from FP64 links (GSOA64, or GAOS64: PyQuda's own), packed;
+// entry q of each array is parity par0 + q's buffer: A (CSOA64), its inverse
+// (CSOA64) and the inverse in FP32 (CSOA32; only beside Ainv64); null: not wanted
+struct CloverOut {
+  void *A64[2] = {nullptr, nullptr}, *Ainv64[2] = {nullptr, nullptr}, *Ainv32[2] = {nullptr, nullptr};
+  int par0 = 0;
+  int *bad = nullptr;  // counts blocks with a zero pivot
+};
+void launch_clover_build(int gkind, const Geom &g, const void *gauge, int nparities, double coeff, const CloverOut &o,
+                         cudaStream_t s);
 // out = C in for a packed clover C (AOS64 or SOA64 spinors)
 void launch_clover_apply(int kind, int Vh, const void *c64, const void *in, void *out, cudaStream_t s);
 size_t clover_bytes(int ckind, int Vh);

@@ -69,7 +69,11 @@ void clover_dslash_noalloc(void *out, const void *in, const void *gauge, const i
   QCU_CUDA(cudaDeviceSynchronize());
   QCU_CUDA(cudaMemsetAsync(slot.bad, 0, sizeof(int), s));  // the counter must start at zero
   // clover of the output parity with qcu's unit normalisation, inverted into the scratch
-  launch_clover_build(g, gauge, parity, 1.0, nullptr, slot.clover, slot.bad, s);
+  CloverOut o;
+  o.par0 = parity;
+  o.Ainv64[0] = slot.clover;
+  o.bad = slot.bad;
+  launch_clover_build(GAOS64, g, gauge, 1, 1.0, o, s);
   DslashArgs d;
   d.in = in;
   d.out = out;

@@ -53,13 +53,17 @@ GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, d
       DevBuf bad;
       bad.ensure(sizeof(int));
       QCU_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx.stream));
+      CloverOut o;
+      o.bad = bad.as<int>();
       for (int p = 0; p < 2; p++) {
         G->A64[p].ensure(clover_bytes(CSOA64, Vh));
         G->Ainv64[p].ensure(clover_bytes(CSOA64, Vh));
         G->Ainv32[p].ensure(clover_bytes(CSOA32, Vh));
-        launch_clover_build(G->g, gauge_pyq, p, clover_coeff, G->A64[p].p, G->Ainv64[p].p, bad.as<int>(), ctx.stream);
-        launch_clover_to32(Vh, G->Ainv64[p].p, G->Ainv32[p].p, ctx.stream);
+        o.A64[p] = G->A64[p].p;
+        o.Ainv64[p] = G->Ainv64[p].p;
+        o.Ainv32[p] = G->Ainv32[p].p;
       }
+      launch_clover_build(GSOA64, G->g, G->g64.p, 2, clover_coeff, o, ctx.stream);
       int nbad = 0;
       QCU_CUDA(cudaMemcpyAsync(&nbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
       QCU_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -739,21 +743,35 @@ void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[
   d.parity = parity;
   d.t_bc = 1.0;
   d.a = 1.0;
+  int gkind = GAOS64;
   if (clover && ctx.legacy_clover == nullptr) {  // this device's scratch, reused across calls, never freed
     ctx.legacy_clover = new DevBuf();
     ctx.legacy_bad = new DevBuf();
+    ctx.legacy_gauge = new DevBuf();
   }
-  DevBuf *cl = ctx.legacy_clover, *bad = ctx.legacy_bad;
+  DevBuf *cl = ctx.legacy_clover, *bad = ctx.legacy_bad, *packed = ctx.legacy_gauge;
   if (clover) {
     // qcu builds the clover of the output parity with unit normalisation on
     // every call (src/nccl_clover_dslash.cu:27-61)
     cl->ensure(clover_bytes(CSOA64, g.Vh));
     bad->ensure(sizeof(int));
     QCU_CUDA(cudaMemsetAsync(bad->p, 0, sizeof(int), ctx.stream));
-    launch_clover_build(g, gauge, parity, 1.0, nullptr, cl->p, bad->as<int>(), ctx.stream);
+    // The build reads every link about 18 times and the hop once more: packing
+    // them first makes those reads contiguous.  Without room for the packed
+    // copy both read the caller's records.
+    if (packed->try_ensure(gauge_bytes(GSOA64, g.Vh))) {
+      launch_gauge_pack(GSOA64, g, gauge, packed->p, ctx.stream);
+      d.gauge = packed->p;
+      gkind = GSOA64;
+    }
+    CloverOut o;
+    o.par0 = parity;
+    o.Ainv64[0] = cl->p;
+    o.bad = bad->as<int>();
+    launch_clover_build(gkind, g, d.gauge, 1, 1.0, o, ctx.stream);
     d.clover = cl->p;
   }
-  launch_dslash(AOS64, GAOS64, CSOA64, g, d, ctx, ctx.stream);
+  launch_dslash(AOS64, gkind, CSOA64, g, d, ctx, ctx.stream);
   QCU_CUDA(cudaStreamSynchronize(ctx.stream));
   if (clover) {
     int nbad = 0;

@@ -406,3 +406,24 @@ def test_dslashQcu_16_byte_aligned_buffers(q):
         assert q.last_error()[0] == 0
         assert rel(host(pout).reshape(ref.shape), ref) <= 1e-13
         assert np.isnan(host(dst)[shift + n:]).all() and np.isnan(host(dst)[:shift]).all()
+
+
+@pytest.mark.parametrize("latt", [[2, 2, 2, 2], [6, 3, 1, 5], [10, 2, 6, 4]])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_clover_term_on_ragged_lattices(q, latt, shift):
+    """The clover build (32 sites a block, neighbours two steps away) on 8, 45 and 240 sites per parity with extents
+    of 1, 2 and 3, on links read from the packed copy, with spinors aligned to 32 and to 16 bytes only."""
+    import torch
+
+    U, psi = _fields(latt, "smooth", 17)
+    dU = dev(U)
+    n = int(np.prod(O.half_shape(latt)))
+    for p in (0, 1):
+        A = O.clover_build(U, latt, p, 1.0)
+        expect = O.clover_apply(O.clover_invert(A), O.dslash(psi[1 - p], U, latt, p))
+        inp, out = (torch.full((n + 1,), float("nan"), dtype=torch.complex128, device="cuda") for _ in range(2))
+        inp[shift:shift + n] = dev(psi[1 - p]).reshape(-1)
+        q.dslashCloverQcu(out[shift:shift + n], inp[shift:shift + n], dU, q.QcuParam(latt), p)
+        assert q.last_error()[0] == 0
+        assert rel(host(out[shift:shift + n]).reshape(expect.shape), expect) <= 1e-14 * max(np.linalg.cond(A).max(), 10)
+        assert bool(torch.isnan(out[n if shift == 0 else 0].real))

@@ -113,7 +113,7 @@ void ncclBistabCgQcu(void *fermion_out, void *fermion_in, void *gauge, QcuParam 
                23333);
       return;
     }
-    G = gauge_load(gauge, param->lattice_size, 1.0, 0.0);
+    G = gauge_load(gauge, param->lattice_size, 1.0, 0.0, /*fp64_only=*/true);
     SolveParams p;
     p.kappa = 0.125;   // include/define.h:69
     p.tol = 1e-9;      // include/define.h:68, absolute on ||r||^2

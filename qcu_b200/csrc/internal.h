@@ -176,7 +176,8 @@ void launch_axpby(int kind, int Vh, double a, void *x, float *xn, double b, void
 void launch_dots(int kind, int Vh, void *a, float *an, void *b, float *bn, Context &ctx, cudaStream_t s);
 
 // gauge: PyQuda complex128 [4][2][Vh][3][3] -> reconstruct-12 internal storage
-void launch_gauge_pack(int gkind, const Geom &g, const void *pyq, void *out, cudaStream_t s);
+// in GSOA64, GSOA32 and GSOA16 (null: not wanted), in one pass over the links
+void launch_gauge_pack(const Geom &g, const void *pyq, void *out64, void *out32, void *out16, cudaStream_t s);
 size_t gauge_bytes(int gkind, int Vh);
 
 // clover: build A = 1 - coeff/8 sum g_mu g_nu (Q - Q^+) on parities par0 ..

@@ -30,7 +30,7 @@ int kind_of_precision(int prec) {
 static int gkind_of(int kind) { return kind == SOA64 ? GSOA64 : (kind == SOA32 ? GSOA32 : GSOA16); }
 static int ckind_of(int kind) { return kind == SOA64 ? CSOA64 : CSOA32; }
 
-GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, double clover_coeff) {
+GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, double clover_coeff, bool fp64_only) {
   require(gauge_pyq != nullptr, "gauge pointer is null");
   require(t_bc == 1.0 || t_bc == -1.0, "t boundary must be +1 or -1");
   Context &ctx = context();
@@ -42,11 +42,11 @@ GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, d
     G->t_bc = t_bc;
     const int Vh = G->g.Vh;
     G->g64.ensure(gauge_bytes(GSOA64, Vh));
-    G->g32.ensure(gauge_bytes(GSOA32, Vh));
-    G->g16.ensure(gauge_bytes(GSOA16, Vh));
-    launch_gauge_pack(GSOA64, G->g, gauge_pyq, G->g64.p, ctx.stream);
-    launch_gauge_pack(GSOA32, G->g, gauge_pyq, G->g32.p, ctx.stream);
-    launch_gauge_pack(GSOA16, G->g, gauge_pyq, G->g16.p, ctx.stream);
+    if (!fp64_only) {
+      G->g32.ensure(gauge_bytes(GSOA32, Vh));
+      G->g16.ensure(gauge_bytes(GSOA16, Vh));
+    }
+    launch_gauge_pack(G->g, gauge_pyq, G->g64.p, G->g32.p, G->g16.p, ctx.stream);
     if (clover_coeff != 0.0) {
       G->has_clover = true;
       G->clover_coeff = clover_coeff;
@@ -729,6 +729,8 @@ void handle_mat(GaugeHandle &G, void *out, const void *in, double kappa, int use
 }
 
 // ---------------------------------------------------------------- legacy direct path
+static constexpr int LEGACY_PACK_VH = 32768;  // 16^4, 38 MB of links
+
 void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[4], int parity, int clover) {
   require(out && in && gauge, "dslash: null pointer argument");
   require(parity == 0 || parity == 1, "parity must be 0 or 1");
@@ -757,10 +759,11 @@ void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[
     bad->ensure(sizeof(int));
     QCU_CUDA(cudaMemsetAsync(bad->p, 0, sizeof(int), ctx.stream));
     // The build reads every link about 18 times and the hop once more: packing
-    // them first makes those reads contiguous.  Without room for the packed
-    // copy both read the caller's records.
-    if (packed->try_ensure(gauge_bytes(GSOA64, g.Vh))) {
-      launch_gauge_pack(GSOA64, g, gauge, packed->p, ctx.stream);
+    // them first makes those reads contiguous.  It pays where the records do
+    // not stay in L2: 24^3 x 48 569 us a call against 629, 16^4 102 us both.  Without room for the packed copy both read
+    // the caller's records.
+    if (g.Vh > LEGACY_PACK_VH && packed->try_ensure(gauge_bytes(GSOA64, g.Vh))) {
+      launch_gauge_pack(g, gauge, packed->p, nullptr, nullptr, ctx.stream);
       d.gauge = packed->p;
       gkind = GSOA64;
     }

@@ -23,7 +23,9 @@ struct GaugeHandle {
   }
 };
 
-GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, double clover_coeff);
+// fp64_only: only the FP64 links, for a handle that no reduced-precision operator will see
+GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, double clover_coeff,
+                        bool fp64_only = false);
 
 struct SolveParams {
   double kappa = 0.125;

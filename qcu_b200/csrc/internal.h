@@ -154,6 +154,17 @@ enum RedKind { RED_NONE = 0, RED_DOT_RT = 1, RED_TS_TT = 2, RED_NORM = 3 };
 void launch_dslash(int kind, int gkind, int ckind, const Geom &g, const DslashArgs &a, Context &ctx,
                    cudaStream_t s);
 
+// out = M in on PyQuda-layout full spinors, M = A - kappa D (both parities); in
+// and out must not overlap.  gauge: GSOA64; A0, A1: the clover term of the even
+// and odd sites (CSOA64), or null for A = 1
+struct MatArgs {
+  const void *in = nullptr;
+  void *out = nullptr;
+  const void *gauge = nullptr, *A0 = nullptr, *A1 = nullptr;
+  double kappa = 0.0, t_bc = 1.0;
+};
+void launch_mat(const Geom &g, const MatArgs &a, cudaStream_t s);
+
 // the vectors of one BiCGSTAB solve: r..t and the partial solution x in the
 // inner precision, x64/r64 the FP64 solution and true residual
 struct VecSet {

@@ -659,6 +659,14 @@ SolveInfo solve(GaugeHandle &G, void *x_pyq, const void *b_pyq, const SolveParam
 }
 
 // ---------------------------------------------------------------- operators on a handle
+// The FP64 operators read and write the caller's PyQuda-layout spinors directly
+// (one pass each way less); a call whose output overlaps its input goes through
+// the internal copies instead.
+static bool overlap(const void *a, const void *b, size_t bytes) {
+  const char *p = static_cast<const char *>(a), *q = static_cast<const char *>(b);
+  return p < q + bytes && q < p + bytes;
+}
+
 void handle_dslash(GaugeHandle &G, void *out, const void *in, int par, int use_clover, int precision) {
   require(out && in, "dslash: null spinor pointer");
   require(par == 0 || par == 1, "parity must be 0 or 1");
@@ -667,8 +675,22 @@ void handle_dslash(GaugeHandle &G, void *out, const void *in, int par, int use_c
   const int kind = kind_of_precision(links16 ? 32 : precision);
   Context &ctx = context();
   std::lock_guard<std::mutex> lk(ctx.mu);
-  Workspace &w = workspace();
   const int Vh = G.g.Vh;
+  if (kind == SOA64 && !overlap(out, in, spinor_bytes(AOS64, Vh))) {
+    QCU_CUDA(cudaDeviceSynchronize());
+    DslashArgs d;
+    d.in = in;
+    d.out = out;
+    d.gauge = G.g64.p;
+    d.clover = use_clover ? G.Ainv64[par].p : nullptr;
+    d.parity = par;
+    d.t_bc = G.t_bc;
+    d.a = 1.0;
+    launch_dslash(AOS64, GSOA64, CSOA64, G.g, d, ctx, ctx.stream);
+    QCU_CUDA(cudaStreamSynchronize(ctx.stream));
+    return;
+  }
+  Workspace &w = workspace();
   w.aux.alloc(SOA64, Vh);
   w.tmp64.alloc(SOA64, Vh);
   w.r.alloc(kind, Vh);
@@ -706,12 +728,26 @@ void handle_mat(GaugeHandle &G, void *out, const void *in, double kappa, int use
   require(!use_clover || G.has_clover, "mat: no clover term loaded");
   Context &ctx = context();
   std::lock_guard<std::mutex> lk(ctx.mu);
-  Workspace &w = workspace();
   const int Vh = G.g.Vh;
+  const size_t half = spinor_bytes(AOS64, Vh);
+  if (!overlap(out, in, 2 * half)) {
+    QCU_CUDA(cudaDeviceSynchronize());
+    MatArgs m;
+    m.in = in;
+    m.out = out;
+    m.gauge = G.g64.p;
+    m.A0 = use_clover ? G.A64[0].p : nullptr;
+    m.A1 = use_clover ? G.A64[1].p : nullptr;
+    m.kappa = kappa;
+    m.t_bc = G.t_bc;
+    launch_mat(G.g, m, ctx.stream);
+    QCU_CUDA(cudaStreamSynchronize(ctx.stream));
+    return;
+  }
+  Workspace &w = workspace();
   for (Spinor *q : {&w.be, &w.bo, &w.tmp64, &w.aux}) q->alloc(SOA64, Vh);
   QCU_CUDA(cudaDeviceSynchronize());
   Dsl d64{G, ctx, SOA64};
-  const size_t half = spinor_bytes(AOS64, Vh);
   launch_convert(AOS64, SOA64, Vh, in, nullptr, w.be.data.p, nullptr, ctx.stream);
   launch_convert(AOS64, SOA64, Vh, static_cast<const char *>(in) + half, nullptr, w.bo.data.p, nullptr, ctx.stream);
   for (int p = 0; p < 2; p++) {
@@ -775,10 +811,10 @@ void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[
     d.clover = cl->p;
   }
   launch_dslash(AOS64, gkind, CSOA64, g, d, ctx, ctx.stream);
+  int nbad = 0;
+  if (clover) QCU_CUDA(cudaMemcpyAsync(&nbad, bad->p, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
   QCU_CUDA(cudaStreamSynchronize(ctx.stream));
   if (clover) {
-    int nbad = 0;
-    QCU_CUDA(cudaMemcpy(&nbad, bad->p, sizeof(int), cudaMemcpyDeviceToHost));
     require(nbad == 0, "clover term is singular on " + std::to_string(nbad) + " site blocks");
   }
 }

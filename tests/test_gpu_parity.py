@@ -427,3 +427,32 @@ def test_clover_term_on_ragged_lattices(q, latt, shift):
         assert q.last_error()[0] == 0
         assert rel(host(out[shift:shift + n]).reshape(expect.shape), expect) <= 1e-14 * max(np.linalg.cond(A).max(), 10)
         assert bool(torch.isnan(out[n if shift == 0 else 0].real))
+
+
+@pytest.mark.parametrize("latt", [[6, 3, 1, 5], [10, 2, 6, 4]])
+@pytest.mark.parametrize("clover", [False, True])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_fp64_operators_on_caller_buffers(q, latt, clover, shift):
+    """dslash and mat in FP64 on 45 and 240 sites per parity, spinors aligned to 32 and to 16 bytes only, and with the
+    output in place of the input and overlapping it by all but one site: the same result, and nothing written beside."""
+    import torch
+
+    U, psi = _fields(latt, "smooth", 19)
+    kappa, c = 0.11, 0.11 if clover else 0.0
+    vh = int(np.prod(O.half_shape(latt))) // 12
+    with q.Gauge(dev(U), latt, t_boundary=-1.0, clover_coeff=c) as G:
+        A = [O.clover_build(U, latt, p, c) for p in (0, 1)] if clover else [None, None]
+        hop = O.dslash(psi[1], U, latt, 0, -1.0)
+        cases = [(psi[1], O.clover_apply(O.clover_invert(A[0]), hop) if clover else hop,
+                  lambda o, i: G.dslash(o, i, 0, clover=clover)),
+                 (psi, O.mfull(psi, U, latt, kappa, -1.0, True, A[0], A[1]), lambda o, i: G.mat(o, i, kappa, clover))]
+        for src, expect, call in cases:
+            n = src.size
+            for to in (n + 24, 0, 12):  # elements between the two: apart, in place, one site on
+                buf = torch.full((2 * n + 60,), float("nan"), dtype=torch.complex128, device="cuda")
+                buf[shift:shift + n] = dev(src).reshape(-1)
+                out = buf[shift + to:shift + to + n]
+                call(out, buf[shift:shift + n])
+                assert rel(host(out).reshape(expect.shape), expect) <= 1e-13
+                assert bool(torch.isnan(buf[shift + to + n:].real).all())
+    assert vh in (45, 240)

@@ -1,7 +1,6 @@
-// Parallel-transport layers of the learned preconditioner: forward,
-// input-gradient (adjoint) and weight-gradient kernels, the training loss
-// and an Adam step.  FP32 arithmetic; weights FP32 (training) or bf16
-// (inference).  See nn.h for the layer definition.
+// Parallel-transport layers of the learned preconditioner: the forward FMA
+// kernel and an Adam step (loss and gradient: nn_train.cu).  FP32 arithmetic;
+// bf16 weights.  See nn.h for the layer definition.
 #include <cuda_bf16.h>
 
 #include "nn.h"
@@ -11,12 +10,8 @@ namespace qcu {
 using F2 = float2;
 
 __device__ __forceinline__ F2 cmul(F2 a, F2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
-__device__ __forceinline__ F2 cmulc(F2 a, F2 b) {  // a * conj(b)
-  return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
-}
 __device__ __forceinline__ F2 cadd(F2 a, F2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 
-__device__ __forceinline__ int hop_bar(int h) { return h == 0 ? 0 : (h & 1 ? h + 1 : h - 1); }
 
 // neighbour of site s (parity par) in direction mu, step +-1; also whether
 // the hop crosses the t boundary
@@ -90,18 +85,8 @@ __device__ __forceinline__ bool transport(const Geom &g, const PtcArgs &a, const
 template <int CIN, int COUT>
 __device__ __forceinline__ void load_weights(const PtcArgs &a, F2 *W) {
   for (int k = threadIdx.x; k < NN_HOPS * COUT * CIN; k += blockDim.x) {
-    const int h = k / (COUT * CIN), ab = k % (COUT * CIN), ao = ab / CIN, bi = ab % CIN;
-    // adjoint: W'[h][a][b] = conj(W[hbar][b][a]) from a [9][CIN][COUT] source
-    const int src = a.adjoint ? (hop_bar(h) * CIN + bi) * COUT + ao : k;
-    F2 w;
-    if (a.w) {
-      w = a.w[src];
-    } else {
-      const uint32_t q = a.w16[src];
-      w = make_float2(__uint_as_float(q << 16), __uint_as_float(q & 0xffff0000u));
-    }
-    if (a.adjoint) w.y = -w.y;
-    W[k] = w;
+    const uint32_t q = a.w16[k];
+    W[k] = make_float2(__uint_as_float(q << 16), __uint_as_float(q & 0xffff0000u));
   }
 }
 
@@ -131,7 +116,7 @@ __global__ void __launch_bounds__(128) k_ptc(Geom g, PtcArgs a) {
 #pragma unroll
   for (int o = 0; o < COUT; o++)
 #pragma unroll
-    for (int c = 0; c < 3; c++) acc[o][c] = a.accumulate ? out[o * 3 + c] : make_float2(0.f, 0.f);
+    for (int c = 0; c < 3; c++) acc[o][c] = make_float2(0.f, 0.f);
   for (int h = 0; h < NN_HOPS; h++) {
     F2 v[CIN][3];
     if (!transport<CIN>(g, a, in_sample, s, par, h, v)) continue;
@@ -148,81 +133,6 @@ __global__ void __launch_bounds__(128) k_ptc(Geom g, PtcArgs a) {
   for (int o = 0; o < COUT; o++)
 #pragma unroll
     for (int c = 0; c < 3; c++) out[o * 3 + c] = acc[o][c];
-}
-
-// weight gradient: every lane runs the same hop loop (zeros where a hop does
-// not apply) so the warp reductions stay converged
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_ptc_wgrad(Geom g, PtcArgs a, F2 *grad) {
-  __shared__ F2 sg[NN_HOPS * COUT * CIN];
-  for (int k = threadIdx.x; k < NN_HOPS * COUT * CIN; k += blockDim.x) sg[k] = make_float2(0.f, 0.f);
-  __syncthreads();
-  int b = 0, par = 0, s = 0;
-  const bool active = decode(g, a, blockIdx.x * (long long)blockDim.x + threadIdx.x, b, par, s);
-  F2 d[COUT][3];
-  const float2 *in_sample = a.in + (size_t)b * 2 * g.Vh * CIN * 3;
-  if (active) {
-    const F2 *dp = a.out + (((size_t)b * 2 + par) * g.Vh + s) * COUT * 3;
-#pragma unroll
-    for (int o = 0; o < COUT; o++)
-#pragma unroll
-      for (int c = 0; c < 3; c++) d[o][c] = dp[o * 3 + c];
-  }
-  const int lane = threadIdx.x & 31;
-  for (int h = 0; h < NN_HOPS; h++) {
-    F2 v[CIN][3];
-    bool ok = active && transport<CIN>(g, a, in_sample, s, par, h, v);
-    if (!ok) {
-#pragma unroll
-      for (int bi = 0; bi < CIN; bi++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) v[bi][c] = make_float2(0.f, 0.f);
-    }
-    if (!__any_sync(0xffffffffu, ok)) continue;
-#pragma unroll
-    for (int o = 0; o < COUT; o++)
-#pragma unroll
-      for (int bi = 0; bi < CIN; bi++) {
-        F2 q = make_float2(0.f, 0.f);
-        if (ok) {
-#pragma unroll
-          for (int c = 0; c < 3; c++) q = cadd(q, cmulc(d[o][c], v[bi][c]));
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-          q.x += __shfl_xor_sync(0xffffffffu, q.x, off);
-          q.y += __shfl_xor_sync(0xffffffffu, q.y, off);
-        }
-        if (lane == 0) {
-          F2 *t = &sg[(h * COUT + o) * CIN + bi];
-          atomicAdd(&t->x, q.x);
-          atomicAdd(&t->y, q.y);
-        }
-      }
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < NN_HOPS * COUT * CIN; k += blockDim.x) {
-    atomicAdd(&grad[k].x, sg[k].x);
-    atomicAdd(&grad[k].y, sg[k].y);
-  }
-}
-
-// delta = (o - e) / (|e|^2 B), loss[i] += |o - e|^2 / |e|^2 over the odd sites
-__global__ void k_nn_loss(Geom g, int B, const F2 *o, const F2 *e, const float *enorm2, F2 *delta, float *loss) {
-  const long long n = (long long)B * g.Vh;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n; idx += (long long)gridDim.x * blockDim.x) {
-    const int b = (int)(idx / g.Vh), s = (int)(idx % g.Vh);
-    const size_t off = (((size_t)b * 2 + 1) * g.Vh + s) * 12;
-    const float inv = 1.f / enorm2[b];
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < 12; k++) {
-      const F2 d = make_float2(o[off + k].x - e[off + k].x, o[off + k].y - e[off + k].y);
-      acc += d.x * d.x + d.y * d.y;
-      delta[off + k] = make_float2(d.x * inv / B, d.y * inv / B);
-    }
-    atomicAdd(&loss[b], acc * inv);
-  }
 }
 
 __global__ void k_adam(int n, float *p, const float *gr, float *m, float *v, uint32_t *p16, float lr, float b1, float b2,
@@ -282,21 +192,6 @@ void launch_ptc(int cin, int cout, const Geom &g, const PtcArgs &a, cudaStream_t
   if (cin == 4 && cout == 16) k_ptc<4, 16><<<blocks, 128, 0, s>>>(g, a);
   else if (cin == 16 && cout == 4) k_ptc<16, 4><<<blocks, 128, 0, s>>>(g, a);
   else throw Error(1, "ptc layer: channels must be 4->16 or 16->4");
-  QCU_CHECK_LAUNCH();
-}
-
-void launch_ptc_wgrad(int cin, int cout, const Geom &g, const PtcArgs &a, float2 *grad, cudaStream_t s) {
-  const long long n = out_sites(g, a);
-  const int blocks = (int)((n + 127) / 128);
-  if (cin == 4 && cout == 16) k_ptc_wgrad<4, 16><<<blocks, 128, 0, s>>>(g, a, grad);
-  else if (cin == 16 && cout == 4) k_ptc_wgrad<16, 4><<<blocks, 128, 0, s>>>(g, a, grad);
-  else throw Error(1, "ptc layer: channels must be 4->16 or 16->4");
-  QCU_CHECK_LAUNCH();
-}
-
-void launch_nn_loss(const Geom &g, int B, const float2 *o, const float2 *e, const float *enorm2, float2 *delta,
-                    float *loss, cudaStream_t s) {
-  k_nn_loss<<<blas_grid(g.Vh * B), BLAS_BLOCK, 0, s>>>(g, B, o, e, enorm2, delta, loss);
   QCU_CHECK_LAUNCH();
 }
 

@@ -8,9 +8,7 @@
 // with T_0 = identity, T_{1+2mu} in(x) = U_mu(x) in(x+mu) and
 // T_{2+2mu} in(x) = U_mu(x-mu)^dag in(x-mu) (t-boundary phase included).
 // W acts on channels only, T on colour only, so the layer commutes with
-// gauge transformations.  The adjoint of T_h is T_hbar (forward <-> backward
-// of the same direction), so the input gradient of a layer is the same
-// kernel run with hops swapped and weights conjugate-transposed.
+// gauge transformations.
 #pragma once
 #include "internal.h"
 
@@ -22,18 +20,15 @@ constexpr int NN_C_IN = 4, NN_C_HID = 16, NN_C_OUT = 4;
 struct PtcArgs {
   const float2 *in = nullptr;   // [B][2][Vh][cin][3]
   float2 *out = nullptr;        // [B][2][Vh][cout][3]
-  const float2 *w = nullptr;    // [9][cout][cin] complex FP32 (or null: use w16)
-  const uint32_t *w16 = nullptr;  // same, as packed bf16 pairs (re, im)
+  const uint32_t *w16 = nullptr;  // [9][cout][cin] complex as packed bf16 pairs (re, im)
   const void *gauge = nullptr;  // GSOA32 packed links
   int B = 1;
   int out_mask = 3;  // bit p: compute output parity p (others are left untouched)
   int in_mask = 3;   // bit q: input is non-zero on parity q (others skipped)
-  int adjoint = 0;   // 1: hops replaced by their adjoints, weights by W^dag (input gradient)
   float t_bc = 1.f;
-  int accumulate = 0;  // 1: out += layer(in)
 };
 
-// forward (or adjoint) layer; cin/cout in {4, 16}
+// forward layer; cin/cout in {4, 16}
 void launch_ptc(int cin, int cout, const Geom &g, const PtcArgs &a, cudaStream_t s);
 // the network's forward pass with bf16 weights on the tensor cores
 // (nn_tc.cu): z64 = N(r64) on odd-parity FP64 site-blocked spinors (SOA64;
@@ -44,13 +39,27 @@ void launch_nn_tc(const Geom &g, const void *gauge16, float t_bc, const uint32_t
                   const void *r64, void *hid16, void *z64, int *err, int sms, cudaStream_t s);
 size_t nn_hid16_bytes(int Vh);
 
-// grad[h][a][b] += sum_x sum_colour delta_a(x) conj((T_h in_b)(x)), over the
-// output parities in a.out_mask (a.out holds delta).  grad: [9][cout][cin] complex FP32.
-void launch_ptc_wgrad(int cin, int cout, const Geom &g, const PtcArgs &a, float2 *grad, cudaStream_t s);
-
-// loss: delta_i = (o_i - e_i) / |e_i|^2 on parity 1, sums_i |o_i - e_i|^2 / |e_i|^2 -> loss[i]
-void launch_nn_loss(const Geom &g, int B, const float2 *o, const float2 *e, const float *enorm2, float2 *delta,
-                    float *loss, cudaStream_t s);
+// Loss and gradient of one batch of odd half spinors r, e (complex128
+// [B][Vh][4][3]): grad = dL/dW* ([9][16][4] then [9][4][16] complex FP32) of
+// L = mean_i |N(r_i) - e_i|^2 / |e_i|^2, enorm[i] = |e_i|^2, and at
+// work[TRAIN_LOSS] the sum of the B losses over B.  fr, fe, a.delta: fields of
+// train_field_bytes each, a.z of eight times that, work of train_part_bytes;
+// a.gauge: GSOA32 links; the rest of a is set here.
+struct TrainArgs {
+  const void *gauge = nullptr;
+  float t_bc = 1.f;
+  int B = 1;
+  const float2 *w1 = nullptr, *w2 = nullptr;
+  float4 *delta = nullptr, *z = nullptr;
+  const float4 *r = nullptr, *e = nullptr;
+  const float *enorm = nullptr;
+  double *part_r = nullptr, *part_s = nullptr;
+};
+constexpr int TRAIN_LOSS = 2048 + 32;
+size_t train_field_bytes(int Vh, int B);
+size_t train_part_bytes(int Vh, int B, int sms);
+void launch_train(const Geom &g, TrainArgs a, const void *r, const void *e, float4 *fr, float4 *fe, double *work,
+                  float *enorm, float2 *grad, int sms, cudaStream_t s);
 
 // Adam step on n real parameters; also refreshes the bf16 copy (pairs)
 void launch_adam(int n, float *p, const float *grad, float *m, float *v, uint32_t *p16, float lr, float b1, float b2,

@@ -19,30 +19,21 @@ constexpr int NN_NPARAM = 2 * (NN_W1 + NN_W2);        // reals
 
 struct NNet {
   DevBuf w, w16, m, v, grad;       // FP32 master, bf16 copy, Adam moments, gradient
-  DevBuf in, hid, out, delta2, delta1, target, enorm, loss;  // work fields (grown to batch x lattice)
+  DevBuf in, hid, out;  // work fields of the FMA layers (grown to the largest lattice)
+  DevBuf tr_r, tr_e, tr_delta, tr_z, tr_work, enorm;  // of a training step (grown to batch x lattice)
   DevBuf err;   // set by the tensor-core layers if a wait timed out
   DevBuf hid16; // hidden field of the tensor-core layers (bf16 pairs)
   int tensor_cores = 1;
   int step = 0;
-  int batch_cap = 0, vh_cap = 0;
   float2 *w1() const { return w.as<float2>(); }
   float2 *w2() const { return w.as<float2>() + NN_W1; }
   uint32_t *w16_1() const { return w16.as<uint32_t>(); }
   uint32_t *w16_2() const { return w16.as<uint32_t>() + NN_W1; }
-  void ensure(int B, int Vh) {
-    if (B <= batch_cap && Vh <= vh_cap) return;
-    batch_cap = std::max(B, batch_cap);
-    vh_cap = std::max(Vh, vh_cap);
-    const size_t f4 = (size_t)batch_cap * 2 * vh_cap * NN_C_IN * 3 * sizeof(float2);
-    const size_t f16 = (size_t)batch_cap * 2 * vh_cap * NN_C_HID * 3 * sizeof(float2);
+  void ensure(int Vh) {
+    const size_t f4 = (size_t)2 * Vh * NN_C_IN * 3 * sizeof(float2);
     in.ensure(f4);
     out.ensure(f4);
-    target.ensure(f4);
-    delta2.ensure(f4);
-    hid.ensure(f16);
-    delta1.ensure(f16);
-    enorm.ensure(batch_cap * sizeof(float));
-    loss.ensure(batch_cap * sizeof(float));
+    hid.ensure(f4 / NN_C_IN * NN_C_HID);
   }
 };
 
@@ -93,30 +84,23 @@ void nn_set(NNet &n, const float *host) {
   QCU_CUDA(cudaStreamSynchronize(ctx.stream));
 }
 
-// N(in) for B samples whose odd halves are in n.in; result in n.out (odd halves).
-// bf16 = true: inference weights; false: FP32 master weights (training)
-static void forward(NNet &n, const GaugeHandle &G, int B, bool bf16, cudaStream_t s) {
+// N(in) by the FMA layers (bf16 weights) for the odd half in n.in; result in n.out (odd half)
+static void forward(NNet &n, const GaugeHandle &G, cudaStream_t s) {
   PtcArgs a;
   a.gauge = G.g32.p;
   a.t_bc = (float)G.t_bc;
-  a.B = B;
   a.in = n.in.as<float2>();
   a.out = n.hid.as<float2>();
   a.in_mask = 2;
   a.out_mask = 3;
-  if (bf16) a.w16 = n.w16_1();
-  else a.w = n.w1();
+  a.w16 = n.w16_1();
   launch_ptc(NN_C_IN, NN_C_HID, G.g, a, s);
-  PtcArgs b2 = a;
-  b2.in = n.hid.as<float2>();
-  b2.out = n.out.as<float2>();
-  b2.in_mask = 3;
-  b2.out_mask = 2;
-  b2.w = nullptr;
-  b2.w16 = nullptr;
-  if (bf16) b2.w16 = n.w16_2();
-  else b2.w = n.w2();
-  launch_ptc(NN_C_HID, NN_C_OUT, G.g, b2, s);
+  a.in = n.hid.as<float2>();
+  a.out = n.out.as<float2>();
+  a.in_mask = 3;
+  a.out_mask = 2;
+  a.w16 = n.w16_2();
+  launch_ptc(NN_C_HID, NN_C_OUT, G.g, a, s);
 }
 
 // z = N(r) on odd-parity SOA64 spinors (z may be r): the tensor-core layers,
@@ -130,7 +114,7 @@ static void apply_soa64(NNet &n, const GaugeHandle &G, const void *r64, void *z6
     return;
   }
   launch_soa64_to_nn(Vh, r64, n.in.as<float2>(), s);
-  forward(n, G, 1, true, s);
+  forward(n, G, s);
   launch_nn_to_soa64(Vh, n.out.as<float2>(), z64, s);
 }
 
@@ -149,7 +133,7 @@ void nn_apply_pyq(NNet &n, const GaugeHandle &G, void *out, const void *in) {
   Context &ctx = context();
   std::lock_guard<std::mutex> lk(ctx.mu);
   const int Vh = G.g.Vh;
-  if (!n.tensor_cores) n.ensure(1, Vh);  // the FMA layers' work fields
+  if (!n.tensor_cores) n.ensure(Vh);  // the FMA layers' work fields
   QCU_CUDA(cudaDeviceSynchronize());
   // complex128 -> FP64 blocked layout, the network, and back
   Spinor &t = stage();
@@ -168,60 +152,30 @@ double nn_train_step(NNet &n, const GaugeHandle &G, const void *r, const void *e
   std::lock_guard<std::mutex> lk(ctx.mu);
   const int Vh = G.g.Vh;
   cudaStream_t s = ctx.stream;
-  n.ensure(B, Vh);
+  const size_t field = train_field_bytes(Vh, B);
+  n.tr_r.ensure(field);
+  n.tr_e.ensure(field);
+  n.tr_delta.ensure(field);
+  n.tr_z.ensure(8 * field);
+  n.tr_work.ensure(train_part_bytes(Vh, B, ctx.sms));
+  n.enorm.ensure(B * sizeof(float));
   QCU_CUDA(cudaDeviceSynchronize());
-  // inputs: odd slabs of samples b (parity 0 slabs are never read: in_mask = 2)
-  Spinor &t = stage();
-  t.alloc(SOA64, Vh);
-  const size_t half = spinor_bytes(AOS64, Vh);
-  std::vector<float> enorm(B);
-  for (int b = 0; b < B; b++) {
-    const char *rb = static_cast<const char *>(r) + b * half;
-    const char *eb = static_cast<const char *>(e) + b * half;
-    launch_convert(AOS64, SOA64, Vh, rb, nullptr, t.data.p, nullptr, s);
-    launch_soa64_to_nn(Vh, t.data.p, n.in.as<float2>() + (size_t)b * 2 * Vh * 12, s);
-    launch_convert(AOS64, SOA64, Vh, eb, nullptr, t.data.p, nullptr, s);
-    launch_soa64_to_nn(Vh, t.data.p, n.target.as<float2>() + (size_t)b * 2 * Vh * 12, s);
-    launch_dots(SOA64, Vh, t.data.p, nullptr, t.data.p, nullptr, ctx, s);
-    QCU_CUDA(cudaMemcpyAsync(ctx.st_host, ctx.st, sizeof(SolverState), cudaMemcpyDeviceToHost, s));
-    QCU_CUDA(cudaStreamSynchronize(s));
-    enorm[b] = (float)ctx.st_host->sums[2];
-    require(enorm[b] > 0.f, "training target with zero norm");
-  }
-  QCU_CUDA(cudaMemcpyAsync(n.enorm.p, enorm.data(), B * sizeof(float), cudaMemcpyHostToDevice, s));
-  QCU_CUDA(cudaMemsetAsync(n.loss.p, 0, B * sizeof(float), s));
-  QCU_CUDA(cudaMemsetAsync(n.grad.p, 0, NN_NPARAM * sizeof(float), s));
-  forward(n, G, B, false, s);
-  launch_nn_loss(G.g, B, n.out.as<float2>(), n.target.as<float2>(), n.enorm.as<float>(), n.delta2.as<float2>(),
-                 n.loss.as<float>(), s);
-  // dL/dW2: delta2 (odd) against the hidden field
-  PtcArgs a;
+  TrainArgs a;
   a.gauge = G.g32.p;
   a.t_bc = (float)G.t_bc;
   a.B = B;
-  a.in = n.hid.as<float2>();
-  a.out = n.delta2.as<float2>();
-  a.in_mask = 3;
-  a.out_mask = 2;
-  launch_ptc_wgrad(NN_C_HID, NN_C_OUT, G.g, a, n.grad.as<float2>() + NN_W1, s);
-  // delta1 = L2^dag delta2 on both parities
-  PtcArgs d = a;
-  d.in = n.delta2.as<float2>();
-  d.out = n.delta1.as<float2>();
-  d.in_mask = 2;
-  d.out_mask = 3;
-  d.adjoint = 1;
-  d.w = n.w2();
-  launch_ptc(NN_C_OUT, NN_C_HID, G.g, d, s);
-  // dL/dW1: delta1 against the input
-  PtcArgs g1 = a;
-  g1.in = n.in.as<float2>();
-  g1.out = n.delta1.as<float2>();
-  g1.in_mask = 2;
-  g1.out_mask = 3;
-  launch_ptc_wgrad(NN_C_IN, NN_C_HID, G.g, g1, n.grad.as<float2>(), s);
-  std::vector<float> loss(B);
-  QCU_CUDA(cudaMemcpyAsync(loss.data(), n.loss.p, B * sizeof(float), cudaMemcpyDeviceToHost, s));
+  a.w1 = n.w1();
+  a.w2 = n.w2();
+  a.delta = n.tr_delta.as<float4>();
+  a.z = n.tr_z.as<float4>();
+  launch_train(G.g, a, r, e, n.tr_r.as<float4>(), n.tr_e.as<float4>(), n.tr_work.as<double>(), n.enorm.as<float>(),
+               n.grad.as<float2>(), ctx.sms, s);
+  std::vector<float> enorm(B);
+  double loss = 0;
+  QCU_CUDA(cudaMemcpyAsync(enorm.data(), n.enorm.p, B * sizeof(float), cudaMemcpyDeviceToHost, s));
+  QCU_CUDA(cudaMemcpyAsync(&loss, n.tr_work.as<double>() + TRAIN_LOSS, sizeof(double), cudaMemcpyDeviceToHost, s));
+  QCU_CUDA(cudaStreamSynchronize(s));
+  for (float x : enorm) require(x > 0.f, "training target with zero norm");  // before the gradient reaches anyone
   if (grad_host) QCU_CUDA(cudaMemcpyAsync(grad_host, n.grad.p, NN_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, s));
   if (lr > 0) {
     n.step++;
@@ -229,9 +183,7 @@ double nn_train_step(NNet &n, const GaugeHandle &G, const void *r, const void *e
                 n.w16.as<uint32_t>(), (float)lr, 0.9f, 0.999f, 1e-8f, n.step, s);
   }
   QCU_CUDA(cudaStreamSynchronize(s));
-  double tot = 0;
-  for (float l : loss) tot += l;
-  return tot / B;
+  return loss / B;
 }
 
 // GCR preconditioner application on FP64 blocked odd spinors: z = N(r)
@@ -241,7 +193,7 @@ void nn_apply_soa64(NNet &n, const GaugeHandle &G, const void *r64, void *z64, c
 
 void nn_prepare(NNet &n, int Vh) {
   if (n.tensor_cores) n.hid16.ensure(nn_hid16_bytes(Vh));
-  else n.ensure(1, Vh);
+  else n.ensure(Vh);
 }
 
 }  // namespace qcu

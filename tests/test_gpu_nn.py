@@ -116,3 +116,28 @@ def test_training_helps_gcr(q):
         i2 = G.invert(x, b, kappa, tol=1e-10, maxiter=4000, solver="gcr", precond=2, nn=net, precision=32,
                       inner_iters=16, gcr_k=8)
         assert i2["status"] == 1 and i2["true_residual"] <= 1e-10
+
+
+@pytest.mark.parametrize("latt,B", [([2, 3, 3, 4], 1), ([6, 3, 1, 5], 7), ([8, 8, 4, 4], 33)])
+def test_gradient_on_ragged_tiles(q, latt, B):
+    """36, 45 and 512 sites per parity (tiles of 32 sites, blocks of 128), a batch of one, an odd one, and one with
+    more tiles (528) than resident blocks; the gradient is FP32 sums of up to 1e5 products: 1e-5."""
+    U = O.gauge_haar(latt, 18)
+    r = O.fermion_gauss((B,) + O.half_shape(latt), 19)
+    e = O.fermion_gauss((B,) + O.half_shape(latt), 20)
+    w = _random_weights(21)
+    net = q.Network()
+    net.set_weights(w)
+    with q.Gauge(dev(U), latt, t_boundary=-1.0) as G:
+        loss, grad = net.train_step(G, dev(r), dev(e), B, 0.0, want_grad=True)
+        loss2, grad2 = net.train_step(G, dev(r), dev(e), B, 0.0, want_grad=True)
+        assert loss == loss2 and np.array_equal(grad, grad2)  # sums in a fixed order
+        e[B // 2] = 0
+        with pytest.raises(q.QcuError):
+            net.train_step(G, dev(r), dev(e), B, 1e-3)
+        assert np.array_equal(net.get_weights(), w)  # a refused batch leaves the weights alone
+    lat = R.Lattice(U, latt, -1.0)
+    e = O.fermion_gauss((B,) + O.half_shape(latt), 20)
+    gref, lref = R.gradient(lat, w.astype(np.float64), r.reshape(B, lat.Vh, 4, 3), e.reshape(B, lat.Vh, 4, 3))
+    assert abs(loss - lref) <= 1e-5 * lref
+    assert rel(grad, gref) < 1e-5

@@ -1,0 +1,96 @@
+// All-reduce, and with it a barrier, over the blocks of a cooperatively
+// launched kernel.  Every block is resident, so every wait ends; the limit on
+// the polls only bounds the damage of a logic error.
+//
+// A block stores its partial sums and counts itself in; one thread of each block
+// watches the counter, and every block then sums all partials in block order.
+// 2.1 us a reduction for 128 blocks (2 and 8 sums alike), against 3.3-4.0 us
+// with a flag per block that one block collects and answers and 3.5-4.2 us when
+// every block watches every other's; watching with acquiring loads, or two
+// loads a turn, costs several us more.
+// The counter goes on rising from launch to launch (modulo 2^32): nothing has
+// to be reset, and launches of different sizes may follow one another.
+#pragma once
+#include "reduce.cuh"
+
+namespace qcu {
+
+constexpr int GRID_RED_BLOCKS = 256;  // at most
+constexpr int GRID_RED_VALUES = 8;    // sums of one reduction, at most
+struct GridRed {
+  unsigned count;  // arrivals
+  unsigned base;   // arrivals of the launches before
+  int failed;      // set when a wait gave up; the host reads and clears the state
+  double part[2][GRID_RED_VALUES][GRID_RED_BLOCKS];
+};
+constexpr unsigned GRID_RED_POLLS = 1u << 21;  // a second or two
+
+struct GridRedShared {
+  double in[32][GRID_RED_VALUES];
+  int ok;
+};
+
+// The sums over the grid of v[0..N) of the threads of every `step`-th warp of
+// each block (the others' are not looked at), into tot (shared memory, N
+// values).  epoch: 1 for the kernel's first reduction, and so on; base: g->base
+// as the kernel found it.  What any thread of any block wrote to global memory
+// before the call can be read after it, with loads that go to L2 (__ldcg).
+// False, in every thread of the block, when the wait gave up: the kernel returns.
+template <int N>
+__device__ __forceinline__ bool grid_allreduce(GridRed *g, unsigned base, unsigned epoch, double (&v)[N], int step,
+                                               double *tot, GridRedShared &sh) {
+  static_assert(N <= GRID_RED_VALUES, "");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (warp % step == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < N; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < N; k++) sh.in[warp][k] = v[k];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    if (lane < N) {
+      double q = 0.0;
+      for (int w = 0; w < nw; w += step) q += sh.in[w][lane];
+      __stcg(&g->part[epoch & 1][lane][blockIdx.x], q);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      atomicAdd(&g->count, 1u);
+      const unsigned target = base + epoch * gridDim.x;
+      unsigned c, polls = 0;
+      int ok = 1;
+      do {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&g->count) : "memory");
+        if (++polls >= GRID_RED_POLLS) {
+          atomicExch(&g->failed, 1);
+          ok = 0;
+          break;
+        }
+      } while ((int)(c - target) < 0);
+      __threadfence();
+      sh.ok = ok;
+    }
+  }
+  __syncthreads();
+  if (!sh.ok) return false;
+  for (int k = warp; k < N; k += nw) {
+    double q = 0.0;
+    for (int i = lane; i < gridDim.x; i += 32) q += __ldcg(&g->part[epoch & 1][k][i]);
+    q = warp_sum(q);
+    if (lane == 0) tot[k] = q;
+  }
+  __syncthreads();
+  return true;
+}
+
+// by one thread of the grid, after its last reduction of the kernel
+__device__ __forceinline__ void grid_red_end(GridRed *g, unsigned base, unsigned epochs) {
+  g->base = base + epochs * gridDim.x;
+}
+
+}  // namespace qcu

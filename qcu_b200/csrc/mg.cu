@@ -27,6 +27,7 @@
 #include <memory>
 #include <vector>
 
+#include "gridbar.cuh"
 #include "mg.h"
 
 namespace qcu {
@@ -367,20 +368,6 @@ __global__ void __launch_bounds__(MG_MAXBLOCK) k_mg_build(MGGeom m, GaugeView<GS
 }
 
 // ---------------------------------------------------------------- coarse solve on the device
-// BiCGSTAB on A_c with its scalars on the device: every kernel of an
-// iteration reads them from CState, one-block finalize kernels update them,
-// and a conditional WHILE node of a CUDA graph repeats the iteration until
-// `done` (converged, iteration cap, breakdown) -- no host round trip.
-struct CState {
-  double2 rho_prev, rho, alpha, omega;
-  double bb, rr;
-  int it, done, status;
-  unsigned guard;
-  long long total_it;      // iterations summed over the solves since the last reset
-  long long total_passes;  // passes of the WHILE body, likewise
-};
-enum CFin { CFIN_INIT = 0, CFIN_ALPHA = 1, CFIN_OMEGA = 2, CFIN_ITER = 3 };
-
 __device__ __forceinline__ double2 cmul2(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -391,185 +378,263 @@ __device__ __forceinline__ double2 cdiv2(double2 a, double2 b) {
 
 constexpr int CAPPLY_WARPS = 8;
 
+// the entries [jp0, jp1) column pairs of one row of A_c times x (xin: the nine
+// blocks' inputs); Yb: the aggregate's matrix at this row (in shared memory when SHARED)
+template <bool SHARED>
+__device__ __forceinline__ float2 mg_row(const float4 *Yb, int nc, const float2 *xin, int jp0, int jp1) {
+  float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
+#pragma unroll 4
+  for (int jp = jp0; jp < jp1; jp++) {
+    const float4 a = SHARED ? Yb[jp * nc] : __ldg(Yb + (size_t)jp * nc);  // (A[2 jp][row], A[2 jp + 1][row])
+    const float2 x0 = xin[2 * jp], x1 = xin[2 * jp + 1];
+    re0 = fmaf(a.x, x0.x, fmaf(-a.y, x0.y, re0));
+    im0 = fmaf(a.x, x0.y, fmaf(a.y, x0.x, im0));
+    re1 = fmaf(a.z, x1.x, fmaf(-a.w, x1.y, re1));
+    im1 = fmaf(a.z, x1.y, fmaf(a.w, x1.x, im1));
+  }
+  return make_float2(re0 + re1, im0 + im1);
+}
+
 // out = A_c in, one warp per aggregate, lane = row; the neighbours' inputs
-// staged in shared memory.  MODE 1: block partials of <w, out>; MODE 2: of
-// <out, w> and |out|^2 (into part[block * 3 + k]).  Skipped when st says done.
-template <int MODE>
+// staged in shared memory (the set-up check; the solve is k_mg_coarse)
 __global__ void __launch_bounds__(32 * CAPPLY_WARPS) k_mg_capply(MGGeom m, const float4 *Y, const float2 *in,
-                                                               float2 *out, const float2 *w, double *part,
-                                                               const CState *st) {
-  if (st != nullptr && st->done) return;
+                                                               float2 *out) {
   __shared__ float2 xin[CAPPLY_WARPS][9 * 2 * MG_MAXVEC];
-  __shared__ double sh[CAPPLY_WARPS * 3];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int B = blockIdx.x * CAPPLY_WARPS + wib;
   const int nc = m.nc, J = 9 * nc;
-  double v[3] = {0, 0, 0};
-  if (B < m.nblocks) {
-    for (int i = lane; i < J; i += 32) {
-      const int d = i / nc;
-      xin[wib][i] = in[(size_t)mg_cnbr(m, B, d) * nc + (i - d * nc)];
-    }
-    __syncwarp();
-    if (lane < nc) {
-      const float4 *Yb = Y + (size_t)B * (J / 2) * nc + lane;
-      float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
-#pragma unroll 4
-      for (int jp = 0; jp < J / 2; jp++) {
-        const float4 a = __ldg(Yb + (size_t)jp * nc);  // (A[2 jp][row], A[2 jp + 1][row])
-        const float2 x0 = xin[wib][2 * jp], x1 = xin[wib][2 * jp + 1];
-        re0 = fmaf(a.x, x0.x, fmaf(-a.y, x0.y, re0));
-        im0 = fmaf(a.x, x0.y, fmaf(a.y, x0.x, im0));
-        re1 = fmaf(a.z, x1.x, fmaf(-a.w, x1.y, re1));
-        im1 = fmaf(a.z, x1.y, fmaf(a.w, x1.x, im1));
-      }
-      const float2 o = make_float2(re0 + re1, im0 + im1);
-      out[(size_t)B * nc + lane] = o;
-      if (MODE == 1) {
-        const float2 a = w[(size_t)B * nc + lane];
-        v[0] = (double)a.x * o.x + (double)a.y * o.y;
-        v[1] = (double)a.x * o.y - (double)a.y * o.x;
-      } else if (MODE == 2) {
-        const float2 a = w[(size_t)B * nc + lane];
-        v[0] = (double)o.x * a.x + (double)o.y * a.y;
-        v[1] = (double)o.x * a.y - (double)o.y * a.x;
-        v[2] = (double)o.x * o.x + (double)o.y * o.y;
-      }
-    }
+  if (B >= m.nblocks) return;
+  for (int i = lane; i < J; i += 32) {
+    const int d = i / nc;
+    xin[wib][i] = in[(size_t)mg_cnbr(m, B, d) * nc + (i - d * nc)];
   }
-  if (MODE != 0) {
-    mg_block_sum<3>(v, sh);
-    if (threadIdx.x == 0)
-      for (int k = 0; k < 3; k++) part[(size_t)blockIdx.x * 3 + k] = v[k];
-  }
+  __syncwarp();
+  if (lane < nc) out[(size_t)B * nc + lane] = mg_row<false>(Y + (size_t)B * (J / 2) * nc + lane, nc, xin[wib], 0, J / 2);
 }
 
-// x = 0, p = v = 0, r = rt = b; block partials of |b|^2 (slot 2)
-__global__ void __launch_bounds__(MG_RED) k_c_init(int64_t n, const float2 *b, float2 *x, float2 *r, float2 *rt,
-                                                 float2 *p, float2 *v, double *part) {
-  __shared__ double sh[(MG_RED / 32) * 3];
-  double a[3] = {0, 0, 0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 q = b[i];
-    x[i] = p[i] = v[i] = make_float2(0.f, 0.f);
-    r[i] = rt[i] = q;
-    a[2] += (double)q.x * q.x + (double)q.y * q.y;
-  }
-  mg_block_sum<3>(a, sh);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; k++) part[(size_t)blockIdx.x * 3 + k] = a[k];
-}
+struct CState {
+  GridRed red;
+  int status;          // of the last solve
+  long long total_it;  // iterations summed over the solves since the last reset
+};
+struct CoarseArgs {
+  MGGeom m;
+  const float4 *Y;
+  const float2 *b;
+  float2 *x, *r0, *r1, *p0, *p1, *v0, *v1, *t;
+  CState *st;
+  double tol2;
+  int maxit;
+  int apb;  // aggregates a block works on at a time: 1, 2 or 4
+};
 
-// the scalar steps: sums nparts partials, then updates the state (one block)
-__global__ void __launch_bounds__(MG_RED) k_c_fin(CState *st, const double *part, int nparts, int op, double tol2,
-                                                int maxit) {
-  if (op != CFIN_INIT && st->done) return;
-  __shared__ double sh[(MG_RED / 32) * 3];
-  double a[3] = {0, 0, 0};
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x)
-    for (int k = 0; k < 3; k++) a[k] += part[(size_t)i * 3 + k];
-  mg_block_sum<3>(a, sh);
-  if (threadIdx.x != 0) return;
-  const double2 one = make_double2(1, 0);
-  if (op == CFIN_INIT) {
-    st->bb = a[2];
-    st->rr = a[2];
-    st->rho = make_double2(a[2], 0);  // <rt, r> with rt = r = b
-    st->rho_prev = st->alpha = st->omega = one;
-    st->it = 0;
-    st->guard = 0;
-    st->done = !(a[2] > 0);
-    st->status = st->done ? ST_CONVERGED : ST_RUNNING;
-  } else if (op == CFIN_ALPHA) {  // a = <rt, v>
-    const double2 rtv = make_double2(a[0], a[1]);
+// x ~ A_c^-1 b by BiCGSTAB (FP32 vectors, FP64 scalars) from zero, to
+// |r|^2 <= tol2 |b|^2 or maxit iterations, as one cooperative kernel.  Two grid
+// barriers an iteration, after each application of A_c: a block forms the
+// vectors it needs at its aggregates' neighbours itself, from the vectors
+// before the update (which therefore alternate between two buffers) and the
+// scalars, instead of waiting for another block to store them; and <rt, r> and
+// |r|^2 of the new residual r = s - omega t follow from the products of s, t
+// and rt that the second application's reduction carries,
+//   <rt, r> = <rt, s> - omega <rt, t>,   |r|^2 = |s|^2 - |<t, s>|^2 / |t|^2.
+// The 32 warps of a block share the columns of 1, 2 or 4 aggregates (lane =
+// row).  Bound by the latency of its barriers and of A_c's entries from L2
+// (from HBM where A_c is larger; where every block's part fits, it stays in
+// shared memory).  16^3 x 32, 4^4 aggregates, 24 rows: 12.8 us an iteration, 4.3
+// of them the barriers, where nine kernels an iteration took 49 us.
+constexpr int MGC_THREADS = 1024;
+constexpr int MGC_SMEM = 180 * 1024;  // the most a block's matrices may take of its shared memory
+template <bool CACHED>
+__global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
+  extern __shared__ float4 ysm[];  // CACHED: the entries of the block's aggregates
+  __shared__ float2 xin[4][9 * 2 * MG_MAXVEC];
+  __shared__ float2 psum[MGC_THREADS / 32][32];
+  __shared__ int nb[4][9];
+  __shared__ GridRedShared red;
+  __shared__ double tot[8];
+  __shared__ double2 sc[5];  // alpha, omega, beta, beta omega, rho
+  __shared__ int done;
+  const int nc = a.m.nc, J = 9 * nc, P = J / 2;
+  const int tpa = MGC_THREADS / a.apb, wpa = tpa / 32;
+  const int al = threadIdx.x / tpa, lt = threadIdx.x % tpa, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = blockIdx.x * a.apb, stride = gridDim.x * a.apb;
+  const int jp0 = (lt >> 5) * P / wpa, jp1 = ((lt >> 5) + 1) * P / wpa;
+  // the (at most two, as J <= 288 and tpa >= 256) inputs this thread stages: block d, row
+  const int d0 = lt / nc, row0 = lt - d0 * nc, d1 = (lt + tpa) / nc, row1 = lt + tpa - d1 * nc;
+  const unsigned count0 = a.st->red.base;
+  unsigned epoch = 0;
+
+  // A_c times the staged inputs at row lt < nc of aggregate B (every thread calls it)
+  auto apply = [&](int B, bool mine) -> float2 {
+    __syncthreads();
+    if (mine && lane < nc)
+      psum[warp][lane] = CACHED ? mg_row<true>(ysm + (size_t)al * P * nc + lane, nc, xin[al], jp0, jp1)
+                                : mg_row<false>(a.Y + (size_t)B * P * nc + lane, nc, xin[al], jp0, jp1);
+    __syncthreads();
+    float2 o = make_float2(0.f, 0.f);
+    if (mine && lt < nc)
+      for (int w = 0; w < wpa; w++) o = make_float2(o.x + psum[al * wpa + w][lt].x, o.y + psum[al * wpa + w][lt].y);
+    return o;
+  };
+  auto neighbours = [&](int B) {
+    if (B < a.m.nblocks && lt < 9) nb[al][lt] = mg_cnbr(a.m, B, lt);
+  };
+
+  double v1[1] = {0.0}, v2[2], v8[8];
+  for (int base = first; base < a.m.nblocks; base += stride) {
+    const int B = base + al;
+    if (B < a.m.nblocks && lt < nc) {
+      const float2 q = a.b[(size_t)B * nc + lt];
+      a.x[(size_t)B * nc + lt] = make_float2(0.f, 0.f);
+      v1[0] += (double)q.x * q.x + (double)q.y * q.y;
+    }
+  }
+  if constexpr (CACHED) {
+    const int n = min(a.apb, a.m.nblocks - first) * P * nc;
+    for (int i = threadIdx.x; i < n; i += MGC_THREADS) ysm[i] = __ldg(a.Y + (size_t)first * P * nc + i);
+    neighbours(first + al);
+  }
+  bool ok = grid_allreduce<1>(&a.st->red, count0, ++epoch, v1, wpa, tot, red);
+  const double bb = tot[0];
+  int status = ok && bb > 0 ? ST_RUNNING : ST_CONVERGED, it = 0;
+  if (threadIdx.x == 0) {
+    sc[0] = sc[1] = sc[2] = sc[3] = make_double2(0, 0);
+    sc[4] = make_double2(bb, 0.0);  // <rt, r> with rt = r = b
+  }
+  for (; ok && status == ST_RUNNING; it++) {
+    const int cur = it & 1;
+    float2 *rc = cur ? a.r1 : a.r0, *pc = cur ? a.p1 : a.p0, *vc = cur ? a.v1 : a.v0;
+    const float2 *ro = cur ? a.r0 : a.r1, *po = cur ? a.p0 : a.p1, *vo = cur ? a.v0 : a.v1;
+    __syncthreads();
+    float ar = (float)sc[0].x, ai = (float)sc[0].y, wr = (float)sc[1].x, wi = (float)sc[1].y;
+    const float br = (float)sc[2].x, bi = (float)sc[2].y, gr = (float)sc[3].x, gi = (float)sc[3].y;
+    // p = r + beta (p - omega v), r the new residual s - omega t; v = A_c p; <rt, v>
+    v2[0] = v2[1] = 0.0;
+    for (int base = first; base < a.m.nblocks; base += stride) {
+      const int B = base + al;
+      const bool mine = B < a.m.nblocks;
+      if constexpr (!CACHED) {
+        __syncthreads();
+        neighbours(B);
+        __syncthreads();
+      }
+      auto stage = [&](int i, int d, int row) {
+        const size_t e = (size_t)nb[al][d] * nc + row;
+        float2 rn, pn;
+        if (it == 0) {
+          rn = pn = a.b[e];
+        } else {
+          const float2 r = __ldcg(ro + e), q = __ldcg(vo + e), t = __ldcg(a.t + e), p = __ldcg(po + e);
+          const float2 s = make_float2(r.x - ar * q.x + ai * q.y, r.y - ar * q.y - ai * q.x);
+          rn = make_float2(s.x - wr * t.x + wi * t.y, s.y - wr * t.y - wi * t.x);
+          pn = make_float2(rn.x + br * p.x - bi * p.y - gr * q.x + gi * q.y,
+                           rn.y + br * p.y + bi * p.x - gr * q.y - gi * q.x);
+          if (d == 8) {
+            const float2 x = a.x[e];
+            a.x[e] = make_float2(x.x + ar * p.x - ai * p.y + wr * s.x - wi * s.y,
+                                 x.y + ar * p.y + ai * p.x + wr * s.y + wi * s.x);
+          }
+        }
+        xin[al][i] = pn;
+        if (d == 8) {
+          rc[e] = rn;
+          pc[e] = pn;
+        }
+      };
+      if (mine && lt < J) stage(lt, d0, row0);
+      if (mine && lt + tpa < J) stage(lt + tpa, d1, row1);
+      const float2 o = apply(B, mine);
+      if (mine && lt < nc) {
+        const size_t e = (size_t)B * nc + lt;
+        vc[e] = o;
+        const float2 q = a.b[e];
+        v2[0] += (double)q.x * o.x + (double)q.y * o.y;
+        v2[1] += (double)q.x * o.y - (double)q.y * o.x;
+      }
+    }
+    ok = grid_allreduce<2>(&a.st->red, count0, ++epoch, v2, wpa, tot, red);
+    if (!ok) break;
+    const double2 rtv = make_double2(tot[0], tot[1]);
     if (!(rtv.x * rtv.x + rtv.y * rtv.y > 0)) {
-      st->done = 1;
-      st->status = ST_BREAKDOWN;
-    } else {
-      st->alpha = cdiv2(st->rho, rtv);
+      status = ST_BREAKDOWN;
+      break;
     }
-  } else if (op == CFIN_OMEGA) {  // a = <t, s>, |t|^2; omega = 0 when t = 0 (then s = 0 too)
-    st->omega = a[2] > 0 ? make_double2(a[0] / a[2], a[1] / a[2]) : make_double2(0, 0);
-  } else {  // CFIN_ITER: a = <rt, r>, |r|^2 of the new residual
-    st->it++;
-    st->total_it++;
-    st->rr = a[2];
-    st->rho_prev = st->rho;
-    st->rho = make_double2(a[0], a[1]);
-    if (!(a[2] == a[2])) {
-      st->done = 1;
-      st->status = ST_NAN;
-    } else if (a[2] <= tol2 * st->bb) {
-      st->done = 1;
-      st->status = ST_CONVERGED;
-    } else if (st->it >= maxit) {
-      st->done = 1;
-      st->status = ST_MAXITER;
-    } else if (!(st->rho.x * st->rho.x + st->rho.y * st->rho.y > 0) ||
-               !(st->omega.x * st->omega.x + st->omega.y * st->omega.y > 0)) {
-      st->done = 1;
-      st->status = ST_BREAKDOWN;
+    if (threadIdx.x == 0) sc[0] = cdiv2(sc[4], rtv);
+    __syncthreads();
+    ar = (float)sc[0].x, ai = (float)sc[0].y;
+    // s = r - alpha v; t = A_c s; the products of t, s and rt
+#pragma unroll
+    for (int k = 0; k < 8; k++) v8[k] = 0.0;
+    for (int base = first; base < a.m.nblocks; base += stride) {
+      const int B = base + al;
+      const bool mine = B < a.m.nblocks;
+      if constexpr (!CACHED) {
+        __syncthreads();
+        neighbours(B);
+        __syncthreads();
+      }
+      auto stage = [&](int i, int d, int row) {
+        const size_t e = (size_t)nb[al][d] * nc + row;
+        const float2 r = __ldcg(rc + e), q = __ldcg(vc + e);
+        xin[al][i] = make_float2(r.x - ar * q.x + ai * q.y, r.y - ar * q.y - ai * q.x);
+      };
+      if (mine && lt < J) stage(lt, d0, row0);
+      if (mine && lt + tpa < J) stage(lt + tpa, d1, row1);
+      const float2 o = apply(B, mine);
+      if (mine && lt < nc) {
+        const size_t e = (size_t)B * nc + lt;
+        a.t[e] = o;
+        const float2 s = xin[al][8 * nc + lt], q = a.b[e];
+        v8[0] += (double)o.x * s.x + (double)o.y * s.y;  // <t, s>
+        v8[1] += (double)o.x * s.y - (double)o.y * s.x;
+        v8[2] += (double)o.x * o.x + (double)o.y * o.y;  // |t|^2
+        v8[3] += (double)q.x * s.x + (double)q.y * s.y;  // <rt, s>
+        v8[4] += (double)q.x * s.y - (double)q.y * s.x;
+        v8[5] += (double)q.x * o.x + (double)q.y * o.y;  // <rt, t>
+        v8[6] += (double)q.x * o.y - (double)q.y * o.x;
+        v8[7] += (double)s.x * s.x + (double)s.y * s.y;  // |s|^2
+      }
+    }
+    ok = grid_allreduce<8>(&a.st->red, count0, ++epoch, v8, wpa, tot, red);
+    if (!ok) break;
+    if (threadIdx.x == 0) {  // omega = 0 when t = 0 (then s = 0 too)
+      const double it2 = tot[2] > 0 ? 1.0 / tot[2] : 0.0;
+      const double2 w = make_double2(tot[0] * it2, tot[1] * it2);
+      const double2 wt = cmul2(w, make_double2(tot[5], tot[6]));
+      const double2 next = make_double2(tot[3] - wt.x, tot[4] - wt.y);
+      const double rr = fmax(tot[7] - (tot[0] * tot[0] + tot[1] * tot[1]) * it2, 0.0);
+      const double2 beta = cdiv2(cmul2(next, sc[0]), cmul2(sc[4], w));
+      sc[1] = w;
+      sc[2] = beta;
+      sc[3] = cmul2(beta, w);
+      sc[4] = next;
+      done = !(tot[7] == tot[7]) || !(tot[2] == tot[2]) ? ST_NAN
+             : rr <= a.tol2 * bb                         ? ST_CONVERGED
+             : it + 1 >= a.maxit                         ? ST_MAXITER
+             : !(next.x * next.x + next.y * next.y > 0) || !(w.x * w.x + w.y * w.y > 0) ? ST_BREAKDOWN
+                                                                                        : ST_RUNNING;
+    }
+    __syncthreads();
+    status = done;
+    if (status != ST_RUNNING) {  // the last x += alpha p + omega s
+      wr = (float)sc[1].x, wi = (float)sc[1].y;
+      for (int base = first; base < a.m.nblocks; base += stride) {
+        const int B = base + al;
+        if (B < a.m.nblocks && lt < nc) {
+          const size_t e = (size_t)B * nc + lt;
+          const float2 r = __ldcg(rc + e), q = __ldcg(vc + e), p = __ldcg(pc + e), x = a.x[e];
+          const float2 s = make_float2(r.x - ar * q.x + ai * q.y, r.y - ar * q.y - ai * q.x);
+          a.x[e] = make_float2(x.x + ar * p.x - ai * p.y + wr * s.x - wi * s.y,
+                               x.y + ar * p.y + ai * p.x + wr * s.y + wi * s.x);
+        }
+      }
     }
   }
-}
-
-// p = r + beta (p - omega v), beta = (rho / rho_prev) (alpha / omega)
-__global__ void k_c_pupdate(int64_t n, float2 *p, const float2 *r, const float2 *v, const CState *st) {
-  if (st->done) return;
-  const double2 beta = cmul2(cdiv2(st->rho, st->rho_prev), cdiv2(st->alpha, st->omega));
-  const double2 bw = cmul2(beta, st->omega);
-  const float br = (float)beta.x, bi = (float)beta.y, wr = (float)bw.x, wi = (float)bw.y;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 pp = p[i], rr = r[i], vv = v[i];
-    p[i] = make_float2(rr.x + br * pp.x - bi * pp.y - wr * vv.x + wi * vv.y,
-                       rr.y + br * pp.y + bi * pp.x - wr * vv.y - wi * vv.x);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    a.st->status = status;
+    a.st->total_it += it;
+    grid_red_end(&a.st->red, count0, epoch);
   }
-}
-
-// s = r - alpha v (in r)
-__global__ void k_c_supdate(int64_t n, float2 *r, const float2 *v, const CState *st) {
-  if (st->done) return;
-  const float ar = (float)st->alpha.x, ai = (float)st->alpha.y;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 rr = r[i], vv = v[i];
-    r[i] = make_float2(rr.x - ar * vv.x + ai * vv.y, rr.y - ar * vv.y - ai * vv.x);
-  }
-}
-
-// x += alpha p + omega s; r = s - omega t; block partials of <rt, r>, |r|^2
-__global__ void __launch_bounds__(MG_RED) k_c_xrupdate(int64_t n, float2 *x, const float2 *p, float2 *r,
-                                                     const float2 *t, const float2 *rt, const CState *st,
-                                                     double *part) {
-  if (st->done) return;
-  __shared__ double sh[(MG_RED / 32) * 3];
-  const float ar = (float)st->alpha.x, ai = (float)st->alpha.y, wr = (float)st->omega.x, wi = (float)st->omega.y;
-  double a[3] = {0, 0, 0};
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float2 pp = p[i], ss = r[i], tt = t[i], xx = x[i], q = rt[i];
-    x[i] = make_float2(xx.x + ar * pp.x - ai * pp.y + wr * ss.x - wi * ss.y,
-                       xx.y + ar * pp.y + ai * pp.x + wr * ss.y + wi * ss.x);
-    const float2 rn = make_float2(ss.x - wr * tt.x + wi * tt.y, ss.y - wr * tt.y - wi * tt.x);
-    r[i] = rn;
-    a[0] += (double)q.x * rn.x + (double)q.y * rn.y;
-    a[1] += (double)q.x * rn.y - (double)q.y * rn.x;
-    a[2] += (double)rn.x * rn.x + (double)rn.y * rn.y;
-  }
-  mg_block_sum<3>(a, sh);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; k++) part[(size_t)blockIdx.x * 3 + k] = a[k];
-}
-
-// the WHILE node's condition: another pass while not done (at most cap passes)
-__global__ void k_c_cond(CState *st, cudaGraphConditionalHandle h, unsigned cap) {
-  const unsigned g = ++st->guard;
-  st->total_passes++;
-  bool go = st->done == 0;
-  if (go && g >= cap) {
-    st->done = 1;
-    st->status = ST_MAXITER;
-    go = false;
-  }
-  cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
 // ---------------------------------------------------------------- vector kernels
@@ -716,17 +781,12 @@ struct MG {
   DevBuf b, x, r, e1, s, q, tmp;
   std::vector<std::unique_ptr<DevBuf>> Z, W;  // flexible GCR directions
   // coarse FP32 vectors
-  DevBuf cb, cx, cr, crt, cp, cv, ct;
+  DevBuf cb, cx, cr, cr2, cp, cp2, cv, cv2, ct;
   DevBuf cstate;                        // CState of the coarse solve
-  cudaGraphExec_t coarse = nullptr;     // the coarse solve cb -> cx as one graph
-  long long coarse_cycles = 0;          // coarse solves launched since the last reset
   double setup_seconds = 0;
 
   int64_t nfull() const { return (int64_t)2 * m.Vp * 12; }
   int64_t ncoarse() const { return (int64_t)m.nblocks * m.nc; }
-  ~MG() {
-    if (coarse) cudaGraphExecDestroy(coarse);
-  }
 };
 
 namespace {
@@ -785,7 +845,6 @@ void mat(MG &mg, Context &ctx, const double2 *in, double2 *out) {
 
 int capply_grid(const MG &mg) { return (mg.m.nblocks + CAPPLY_WARPS - 1) / CAPPLY_WARPS; }
 
-// out = A_c in (no reduction)
 // out = b - M e on full FP64 vectors in one dslash pass per parity:
 // out_p = kappa D_{p <- 1-p} e_{1-p} + b_p - A_p e_p
 void residual(MG &mg, Context &ctx, const double2 *e, const double2 *b, double2 *out) {
@@ -812,100 +871,52 @@ void residual(MG &mg, Context &ctx, const double2 *e, const double2 *b, double2 
   }
 }
 
+// out = A_c in
 void capply(MG &mg, cudaStream_t st, const float2 *in, float2 *out) {
-  k_mg_capply<0><<<capply_grid(mg), 32 * CAPPLY_WARPS, 0, st>>>(mg.m, mg.Y.as<float4>(), in, out, nullptr, nullptr,
-                                                                nullptr);
+  k_mg_capply<<<capply_grid(mg), 32 * CAPPLY_WARPS, 0, st>>>(mg.m, mg.Y.as<float4>(), in, out);
   QCU_CHECK_LAUNCH();
 }
 
-constexpr int COARSE_KERNELS_PER_PASS = 9;
-
-// The coarse solve cx ~ A_c^-1 cb as a graph: init, then a WHILE node whose
-// body is one BiCGSTAB iteration (FP32 vectors, FP64 scalars in CState) to
-// |r| <= coarse_tol |b| or coarse_maxiter iterations.
-void capture_coarse(MG &mg, Context &ctx) {
-  cudaStream_t st = ctx.stream;
-  const int64_t n = mg.ncoarse();
-  const int gv = mg_grid(n), ga = capply_grid(mg);
-  CState *cs = mg.cstate.as<CState>();
-  double *part = mg.part.as<double>();
-  const double tol2 = mg.p.coarse_tol * mg.p.coarse_tol;
-  const int maxit = mg.p.coarse_maxiter;
-  float2 *b = f32(mg.cb), *x = f32(mg.cx), *r = f32(mg.cr), *rt = f32(mg.crt), *p = f32(mg.cp), *v = f32(mg.cv),
-         *t = f32(mg.ct);
-  const float4 *Y = mg.Y.as<float4>();
-  const auto mode = cudaStreamCaptureModeThreadLocal;
-  const long long before = launch_count();
-  cudaGraph_t g = nullptr;
-  QCU_CUDA(cudaGraphCreate(&g, 0));
-  try {
-    QCU_CUDA(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, mode));
-    k_c_init<<<gv, MG_RED, 0, st>>>(n, b, x, r, rt, p, v, part);
-    QCU_CHECK_LAUNCH();
-    k_c_fin<<<1, MG_RED, 0, st>>>(cs, part, gv, CFIN_INIT, tol2, maxit);
-    QCU_CHECK_LAUNCH();
-    QCU_CUDA(cudaStreamEndCapture(st, &g));
-    size_t nn = 0;
-    QCU_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
-    require(nn == 2, "mg: unexpected coarse-solve init capture");
-    std::vector<cudaGraphNode_t> nodes(nn);
-    QCU_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-    cudaGraphNode_t last = nodes[0];  // the node without dependents (the finalize)
-    for (cudaGraphNode_t nd : nodes) {
-      size_t nd_out = 0;
-      QCU_CUDA(cudaGraphNodeGetDependentNodes(nd, nullptr, &nd_out));
-      if (nd_out == 0) last = nd;
-    }
-    cudaGraphConditionalHandle h;
-    QCU_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t loop;
-    QCU_CUDA(cudaGraphAddNode(&loop, g, &last, 1, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    QCU_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, mode));
-    k_c_pupdate<<<gv, MG_RED, 0, st>>>(n, p, r, v, cs);
-    QCU_CHECK_LAUNCH();
-    k_mg_capply<1><<<ga, 32 * CAPPLY_WARPS, 0, st>>>(mg.m, Y, p, v, rt, part, cs);
-    QCU_CHECK_LAUNCH();
-    k_c_fin<<<1, MG_RED, 0, st>>>(cs, part, ga, CFIN_ALPHA, tol2, maxit);
-    QCU_CHECK_LAUNCH();
-    k_c_supdate<<<gv, MG_RED, 0, st>>>(n, r, v, cs);
-    QCU_CHECK_LAUNCH();
-    k_mg_capply<2><<<ga, 32 * CAPPLY_WARPS, 0, st>>>(mg.m, Y, r, t, r, part, cs);
-    QCU_CHECK_LAUNCH();
-    k_c_fin<<<1, MG_RED, 0, st>>>(cs, part, ga, CFIN_OMEGA, tol2, maxit);
-    QCU_CHECK_LAUNCH();
-    k_c_xrupdate<<<gv, MG_RED, 0, st>>>(n, x, p, r, t, rt, cs, part);
-    QCU_CHECK_LAUNCH();
-    k_c_fin<<<1, MG_RED, 0, st>>>(cs, part, gv, CFIN_ITER, tol2, maxit);
-    QCU_CHECK_LAUNCH();
-    k_c_cond<<<1, 1, 0, st>>>(cs, h, (unsigned)maxit + 2u);
-    QCU_CHECK_LAUNCH();
-    QCU_CUDA(cudaStreamEndCapture(st, &body));
-    QCU_CUDA(cudaGraphInstantiate(&mg.coarse, g, 0));
-  } catch (...) {
-    cudaStreamCaptureStatus csx;
-    if (cudaStreamIsCapturing(st, &csx) == cudaSuccess && csx != cudaStreamCaptureStatusNone) {
-      cudaGraph_t junk;
-      cudaStreamEndCapture(st, &junk);
-    }
-    cudaGetLastError();
-    cudaGraphDestroy(g);
-    set_launch_count(before);
-    throw;
-  }
-  cudaGraphDestroy(g);
-  set_launch_count(before);  // replays are counted from the passes the state records
+// cx ~ A_c^-1 cb on the device
+void coarse_solve(MG &mg, Context &ctx) {
+  CoarseArgs a;
+  a.m = mg.m;
+  a.Y = mg.Y.as<float4>();
+  a.b = f32(mg.cb);
+  a.x = f32(mg.cx);
+  a.r0 = f32(mg.cr);
+  a.r1 = f32(mg.cr2);
+  a.p0 = f32(mg.cp);
+  a.p1 = f32(mg.cp2);
+  a.v0 = f32(mg.cv);
+  a.v1 = f32(mg.cv2);
+  a.t = f32(mg.ct);
+  a.st = mg.cstate.as<CState>();
+  a.tol2 = mg.p.coarse_tol * mg.p.coarse_tol;
+  a.maxit = mg.p.coarse_maxiter;
+  // spread the aggregates over the SMs before a block takes several at a time
+  a.apb = mg.m.nblocks <= ctx.sms ? 1 : (mg.m.nblocks <= 2 * ctx.sms ? 2 : 4);
+  const int grid = std::min(std::min(ctx.sms, GRID_RED_BLOCKS), (mg.m.nblocks + a.apb - 1) / a.apb);
+  // A_c stays in shared memory where every block has one set of aggregates that fits
+  const size_t smem = (size_t)a.apb * (9 * a.m.nc / 2) * a.m.nc * sizeof(float4);
+  const bool cached = smem <= MGC_SMEM && (int64_t)grid * a.apb >= a.m.nblocks;
+  const void *k = cached ? reinterpret_cast<const void *>(k_mg_coarse<true>) : reinterpret_cast<const void *>(k_mg_coarse<false>);
+  if (cached) QCU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MGC_SMEM));
+  void *args[] = {&a};
+  QCU_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(MGC_THREADS), args, cached ? smem : 0, ctx.stream));
+  note_launch(1);
 }
 
-// cx ~ A_c^-1 cb on the device
-void coarse_solve(MG &mg, cudaStream_t st) {
-  QCU_CUDA(cudaGraphLaunch(mg.coarse, st));
-  mg.coarse_cycles++;
+// the state of the coarse solves since the last reset, on the host; throws if a barrier gave up
+CState coarse_state(MG &mg, cudaStream_t st) {
+  CState cs;
+  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, sizeof(CState), cudaMemcpyDeviceToHost, st));
+  QCU_CUDA(cudaStreamSynchronize(st));
+  if (cs.red.failed) {
+    QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, sizeof(CState), st));
+    throw Error(2, "mg: a barrier of the coarse solve timed out");
+  }
+  return cs;
 }
 
 void axpy2(cudaStream_t st, int64_t n, double2 *x, const double2 *y, double2 *r, const double2 *w, C a) {
@@ -947,7 +958,7 @@ void cycle(MG &mg, Context &ctx, const double2 *r, double2 *e) {
   }
   k_mg_restrict<<<m.nblocks, m.bsites, 0, st>>>(m, nv, slabs(mg, rc), f32(mg.cb));
   QCU_CHECK_LAUNCH();
-  coarse_solve(mg, st);
+  coarse_solve(mg, ctx);
   k_mg_prolong<<<m.nblocks, m.bsites, 0, st>>>(m, nv, f32(mg.cx), slabs(mg, e), mg.p.nu_pre > 0 ? 1 : 0);
   QCU_CHECK_LAUNCH();
   if (mg.p.nu_post > 0) smooth(mg, ctx, r, e, mg.p.nu_post, false);
@@ -992,7 +1003,7 @@ MG *mg_create(GaugeHandle &G, double kappa, const MGParams &p) {
     const size_t cfull = (size_t)mg->ncoarse() * sizeof(float2);
     mg->nv.ensure((size_t)m.nvec * mg->nfull() * sizeof(float2));
     mg->Y.ensure((size_t)m.nblocks * 9 * m.nc * m.nc * sizeof(float2));
-    mg->part.ensure((size_t)std::max(MG_RED_GRID * 2 * MG_CHUNK, capply_grid(*mg) * 3) * sizeof(double));
+    mg->part.ensure((size_t)MG_RED_GRID * 2 * MG_CHUNK * sizeof(double));
     mg->cstate.ensure(sizeof(CState));
     QCU_CUDA(cudaMemsetAsync(mg->cstate.p, 0, sizeof(CState), ctx.stream));
     mg->part_h.resize((size_t)MG_RED_GRID * 2 * MG_CHUNK);
@@ -1004,7 +1015,8 @@ MG *mg_create(GaugeHandle &G, double kappa, const MGParams &p) {
       mg->Z.back()->ensure(full);
       mg->W.back()->ensure(full);
     }
-    for (DevBuf *d : {&mg->cb, &mg->cx, &mg->cr, &mg->crt, &mg->cp, &mg->cv, &mg->ct}) d->ensure(cfull);
+    for (DevBuf *d : {&mg->cb, &mg->cx, &mg->cr, &mg->cr2, &mg->cp, &mg->cp2, &mg->cv, &mg->cv2, &mg->ct})
+      d->ensure(cfull);
     // the padding sites of the full vectors stay zero throughout
     for (DevBuf *d : {&mg->b, &mg->x, &mg->r, &mg->e1, &mg->s, &mg->q}) QCU_CUDA(cudaMemsetAsync(d->p, 0, full, ctx.stream));
     for (int k = 0; k < p.gcr_k; k++) {
@@ -1065,7 +1077,6 @@ MG *mg_create(GaugeHandle &G, double kappa, const MGParams &p) {
                                              mg->nv.as<float2>(), mg->Y.as<float2>());
   QCU_CHECK_LAUNCH();
   QCU_CUDA(cudaStreamSynchronize(st));
-  capture_coarse(*mg, ctx);
   mg->setup_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   return mg.release();
 }
@@ -1093,7 +1104,7 @@ void mg_coarse_odd(MG &mg, Context &ctx, const void *r_odd, void *z_odd) {
   k_mg_restrict<<<m.nblocks, m.bsites, 0, st>>>(m, nv, FineVec{{nullptr, const_cast<double2 *>(src)}},
                                                 f32(mg.cb));
   QCU_CHECK_LAUNCH();
-  coarse_solve(mg, st);
+  coarse_solve(mg, ctx);
   k_mg_prolong<<<m.nblocks, m.bsites, 0, st>>>(m, nv, f32(mg.cx), FineVec{{nullptr, static_cast<double2 *>(z_odd)}},
                                                0);
   QCU_CHECK_LAUNCH();
@@ -1118,15 +1129,7 @@ double2 mg_minres_scale(MG &mg, Context &ctx, void *z, void *q, const void *r) {
   return al;
 }
 
-long long mg_take_launches(MG &mg, Context &ctx) {
-  CState cs;
-  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, sizeof(CState), cudaMemcpyDeviceToHost, ctx.stream));
-  QCU_CUDA(cudaStreamSynchronize(ctx.stream));
-  const long long n = 2 * mg.coarse_cycles + COARSE_KERNELS_PER_PASS * cs.total_passes;
-  QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, sizeof(CState), ctx.stream));
-  mg.coarse_cycles = 0;
-  return n;
-}
+void mg_check_coarse(MG &mg, Context &ctx) { coarse_state(mg, ctx.stream); }
 
 double mg_setup_seconds(const MG &mg) { return mg.setup_seconds; }
 
@@ -1150,7 +1153,6 @@ MGInfo mg_solve(MG &mg, void *x_pyq, const void *b_pyq, double tol, int maxiter)
   QCU_CUDA(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double2), st));
   QCU_CUDA(cudaMemcpyAsync(r, b, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
   MGInfo info;
-  mg.coarse_cycles = 0;
   QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, sizeof(CState), st));
   double d[3];
   dots(mg, st, n, b, b, d);
@@ -1225,11 +1227,8 @@ MGInfo mg_solve(MG &mg, void *x_pyq, const void *b_pyq, double tol, int maxiter)
     rr = d[2];
   }
   info.true_residual = std::sqrt(rr / bb);
-  CState cs;
-  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, sizeof(CState), cudaMemcpyDeviceToHost, st));
-  QCU_CUDA(cudaStreamSynchronize(st));
+  const CState cs = coarse_state(mg, st);
   info.coarse_iters = (int)std::min<long long>(cs.total_it, 0x7fffffff);
-  note_launch(2 * mg.coarse_cycles + COARSE_KERNELS_PER_PASS * cs.total_passes);
   for (int par = 0; par < 2; par++)
     launch_convert(SOA64, AOS64, Vh, x + par * half, nullptr, static_cast<char *>(x_pyq) + par * half_pyq, nullptr,
                    st);

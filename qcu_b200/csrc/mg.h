@@ -50,7 +50,7 @@ void mg_coarse_odd(MG &mg, Context &ctx, const void *r_odd, void *z_odd);
 double2 mg_minres_scale(MG &mg, Context &ctx, void *z, void *q, const void *r);
 // throws unless mg was built on G for this kappa, with the clover term iff G has one
 void mg_require_compatible(const MG &mg, const GaugeHandle &G, double kappa, int use_clover);
-// kernels the coarse solves launched since the last call (read from the device)
-long long mg_take_launches(MG &mg, Context &ctx);
+// throws if a barrier of a coarse solve gave up (waits for the stream)
+void mg_check_coarse(MG &mg, Context &ctx);
 
 }  // namespace qcu

@@ -490,7 +490,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
     throw;
   }
   if (inner) cudaGraphExecDestroy(inner);
-  if (pc == 3) note_launch(mg_take_launches(*prm.mg, ctx));
+  if (pc == 3) mg_check_coarse(*prm.mg, ctx);
   if (info.status == ST_RUNNING && info.iterations >= prm.maxiter) info.status = ST_MAXITER;
 }
 

@@ -274,17 +274,18 @@ static void launch_clov(const Geom &g, const DslashArgs &a, Context &ctx, cudaSt
 
 void launch_dslash(int kind, int gkind, int ckind, const Geom &g, const DslashArgs &a, Context &ctx,
                    cudaStream_t s) {
-  // PyQuda-layout spinors whose buffers are all 32-byte aligned take the 32-byte accesses
-  auto al32 = [](const void *p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 31) == 0; };
-  if (kind == AOS64 && gkind == GAOS64 && ckind == CSOA64 && al32(a.in) && al32(a.out) && al32(a.x1) &&
-      al32(a.x2) && al32(a.rt))
-    launch_clov<AOS64W, GAOS64, CSOA64>(g, a, ctx, s);
-  else if (kind == AOS64 && gkind == GAOS64 && ckind == CSOA64) launch_clov<AOS64, GAOS64, CSOA64>(g, a, ctx, s);
-  else if (kind == AOS64 && gkind == GSOA64 && ckind == CSOA64) {
-    // PyQuda-layout spinors on packed links: the hop with or without the inverse clover
-    require(a.x1 == nullptr && a.x2 == nullptr && a.red == RED_NONE, "dslash: no epilogue on this storage combination");
-    const bool wide = al32(a.in) && al32(a.out);
-    if (wide && a.clover) launch_t<AOS64W, GSOA64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
+  if (kind == AOS64 && ckind == CSOA64) {
+    // PyQuda-layout spinors: the hop with or without the inverse clover, on
+    // PyQuda's own links or packed ones; buffers that are 32-byte aligned take
+    // the 32-byte accesses
+    require(a.x1 == nullptr && a.x2 == nullptr && a.red == RED_NONE && a.gate == GATE_ALWAYS && a.a == 1.0,
+            "dslash: no epilogue on PyQuda-layout spinors");
+    const bool wide = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out)) & 31) == 0;
+    if (gkind == GAOS64 && !a.clover) launch_hop_records(g, a.in, a.out, a.gauge, a.parity, a.t_bc, s);
+    else if (gkind == GAOS64 && wide) launch_t<AOS64W, GAOS64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
+    else if (gkind == GAOS64) launch_t<AOS64, GAOS64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
+    else if (gkind != GSOA64) throw Error(1, "dslash: unsupported storage combination");
+    else if (wide && a.clover) launch_t<AOS64W, GSOA64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
     else if (wide) launch_t<AOS64W, GSOA64, CSOA64, false, 0, RED_NONE>(g, a, ctx, s);
     else if (a.clover) launch_t<AOS64, GSOA64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
     else launch_t<AOS64, GSOA64, CSOA64, false, 0, RED_NONE>(g, a, ctx, s);

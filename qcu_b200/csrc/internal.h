@@ -154,6 +154,11 @@ enum RedKind { RED_NONE = 0, RED_DOT_RT = 1, RED_TS_TT = 2, RED_NORM = 3 };
 void launch_dslash(int kind, int gkind, int ckind, const Geom &g, const DslashArgs &a, Context &ctx,
                    cudaStream_t s);
 
+// out(par) = D in on PyQuda-layout half spinors and links (hop_records.cu); in
+// and out must not overlap
+void launch_hop_records(const Geom &g, const void *in, void *out, const void *gauge, int par, double t_bc,
+                        cudaStream_t s);
+
 // out = M in on PyQuda-layout full spinors, M = A - kappa D (both parities); in
 // and out must not overlap.  gauge: GSOA64; A0, A1: the clover term of the even
 // and odd sites (CSOA64), or null for A = 1

@@ -456,3 +456,24 @@ def test_fp64_operators_on_caller_buffers(q, latt, clover, shift):
                 assert rel(host(out).reshape(expect.shape), expect) <= 1e-13
                 assert bool(torch.isnan(buf[shift + to + n:].real).all())
     assert vh in (45, 240)
+
+
+@pytest.mark.parametrize("latt", [[2, 2, 2, 2], [6, 3, 1, 5], [4, 2, 2, 4], [34, 2, 2, 2]])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_dslashQcu_on_partial_warps(q, latt, shift):
+    """The staged hop moves records for 32 sites a warp, four warps a block: 8, 45, 32 and 136 sites per parity, rows
+    that wrap inside a warp's records, links and spinors aligned to 32 and to 16 bytes only."""
+    import torch
+
+    U, psi = _fields(latt, "haar", 23)
+    n, m = int(np.prod(O.half_shape(latt))), U.size
+    links = torch.zeros(m + 1, dtype=torch.complex128, device="cuda")
+    links[shift:shift + m] = dev(U).reshape(-1)
+    for p in (0, 1):
+        src, dst = (torch.full((n + 1,), float("nan"), dtype=torch.complex128, device="cuda") for _ in range(2))
+        src[shift:shift + n] = dev(psi[1 - p]).reshape(-1)
+        q.dslashQcu(dst[shift:shift + n], src[shift:shift + n], links[shift:shift + m], q.QcuParam(latt), p)
+        assert q.last_error()[0] == 0
+        ref = O.dslash(psi[1 - p], U, latt, p)
+        assert rel(host(dst[shift:shift + n]).reshape(ref.shape), ref) <= 1e-13
+        assert bool(torch.isnan(dst[n if shift == 0 else 0].real))

@@ -292,23 +292,24 @@ __device__ __forceinline__ void kb_xrupdate_tile(const BatchArgs &a, const int2 
   double red[3] = {0, 0, 0};
   BTILE_SITES(a, tile, d)
   for (int s = s_begin + threadIdx.x; s < s_end; s += BB) {
-    Cpx<T> p[12], q[12], t[12];
+    // every input first: the vectors are distinct buffers, so no store below feeds a load
+    Cpx<T> p[12], q[12], t[12], rt[12];
     Cpx<TX> x[12];
     spinor_load<K, T>(bview<K>(d, BV_P), s, p);
     spinor_load<K, T>(bview<K>(d, BV_S), s, q);
     spinor_load<XK, TX>(bview<XK>(d, BV_X), s, x);
+    spinor_load<K, T>(bview<K>(d, BV_T), s, t);
+    spinor_load<K, T>(bview<K>(d, BV_RT), s, rt);
 #pragma unroll
     for (int c = 0; c < 12; c++) {
       x[c] += Cpx<TX>((TX)p[c].re, (TX)p[c].im) * ax;
       x[c] += Cpx<TX>((TX)q[c].re, (TX)q[c].im) * wx;
     }
     spinor_store<XK, TX>(bview<XK>(d, BV_X), s, x);
-    spinor_load<K, T>(bview<K>(d, BV_T), s, t);
 #pragma unroll
     for (int c = 0; c < 12; c++) q[c] = q[c] - t[c] * w;
     spinor_store<K, T>(bview<K>(d, BV_R), s, q);
-    spinor_load<K, T>(bview<K>(d, BV_RT), s, p);
-    site_dot<T>(p, q, red[0], red[1]);
+    site_dot<T>(rt, q, red[0], red[1]);
     site_norm2<T>(q, red[2]);
   }
   warp_red_add(wr, tile.x, red);
@@ -561,12 +562,23 @@ __global__ void __launch_bounds__(BB) kb_gcr_update(BatchArgs a, int k) {
 }
 
 // ---------------------------------------------------------------- launchers
-// Grid of a persistent batched kernel: as many blocks as the SMs can hold by
-// thread count (or fewer when the table has fewer tiles); each block then
-// walks the tile table with a stride of the grid.
-static int persistent_grid(const BatchArgs &a, int threads) {
-  const int cap = std::min(BATCH_POST_GRID, std::max(1, a.sms) * std::max(1, 1024 / threads));
+// Grid of a persistent batched kernel: one wave of the blocks that are resident
+// with the kernel's registers and shared memory (or fewer when the table has
+// fewer tiles); each block then walks the tile table with a stride of the grid.
+// (A grid by thread count, 8 blocks an SM where 6 fit, ran its last quarter in a
+// second, mostly empty wave: kb_xrupdate 76 -> 64 us at 12 rhs of 16^3 x 32, its
+// loads all before its stores included.)
+template <typename F>
+static int persistent_grid(const BatchArgs &a, F kernel) {
+  int per_sm = 0;
+  QCU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BB, 0));
+  const int cap = std::min(BATCH_POST_GRID, std::max(1, a.sms) * std::max(1, per_sm));
   return std::max(1, std::min(a.ntiles, cap));
+}
+// the FP64 outer kernels reduce per tile: more blocks than are resident hide
+// that (kb_gcr_multidot 186 us against 234 with one wave)
+static int tile_grid(const BatchArgs &a) {
+  return std::max(1, std::min(a.ntiles, std::min(BATCH_POST_GRID, std::max(1, a.sms) * (1024 / BB))));
 }
 // the hopping kernels: the blocks their registers let reside per SM
 static int dslash_grid(const BatchArgs &a, int per_sm) {
@@ -641,32 +653,32 @@ void launch_bdslash(int kind, int gkind, const BatchArgs &a, const BDslOp &op, c
 }
 
 void launch_bpupdate(int kind, const BatchArgs &a, cudaStream_t s) {
-  if (kind == SOA64) kb_pupdate<SOA64><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else if (kind == SOA16) kb_pupdate<SOA16><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else kb_pupdate<SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);
+  if (kind == SOA64) kb_pupdate<SOA64><<<persistent_grid(a, kb_pupdate<SOA64>), BB, 0, s>>>(a);
+  else if (kind == SOA16) kb_pupdate<SOA16><<<persistent_grid(a, kb_pupdate<SOA16>), BB, 0, s>>>(a);
+  else kb_pupdate<SOA32><<<persistent_grid(a, kb_pupdate<SOA32>), BB, 0, s>>>(a);
   QCU_CHECK_LAUNCH();
 }
 void launch_bsupdate(int kind, const BatchArgs &a, cudaStream_t s) {
-  if (kind == SOA64) kb_supdate<SOA64><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else if (kind == SOA16) kb_supdate<SOA16><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else kb_supdate<SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);
+  if (kind == SOA64) kb_supdate<SOA64><<<persistent_grid(a, kb_supdate<SOA64>), BB, 0, s>>>(a);
+  else if (kind == SOA16) kb_supdate<SOA16><<<persistent_grid(a, kb_supdate<SOA16>), BB, 0, s>>>(a);
+  else kb_supdate<SOA32><<<persistent_grid(a, kb_supdate<SOA32>), BB, 0, s>>>(a);
   QCU_CHECK_LAUNCH();
 }
 void launch_bxrupdate(int kind, const BatchArgs &a, cudaStream_t s) {
-  if (kind == SOA64) kb_xrupdate<SOA64, SOA64><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else if (kind == SOA16) kb_xrupdate<SOA16, SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);  // x in FP32
-  else kb_xrupdate<SOA32, SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);
+  if (kind == SOA64) kb_xrupdate<SOA64, SOA64><<<persistent_grid(a, kb_xrupdate<SOA64, SOA64>), BB, 0, s>>>(a);
+  else if (kind == SOA16) kb_xrupdate<SOA16, SOA32><<<persistent_grid(a, kb_xrupdate<SOA16, SOA32>), BB, 0, s>>>(a);  // x in FP32
+  else kb_xrupdate<SOA32, SOA32><<<persistent_grid(a, kb_xrupdate<SOA32, SOA32>), BB, 0, s>>>(a);
   QCU_CHECK_LAUNCH();
 }
 void launch_binit(int kind, const BatchArgs &a, cudaStream_t s) {
-  if (kind == SOA64) kb_init<SOA64, SOA64><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else if (kind == SOA16) kb_init<SOA16, SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else kb_init<SOA32, SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);
+  if (kind == SOA64) kb_init<SOA64, SOA64><<<persistent_grid(a, kb_init<SOA64, SOA64>), BB, 0, s>>>(a);
+  else if (kind == SOA16) kb_init<SOA16, SOA32><<<persistent_grid(a, kb_init<SOA16, SOA32>), BB, 0, s>>>(a);
+  else kb_init<SOA32, SOA32><<<persistent_grid(a, kb_init<SOA32, SOA32>), BB, 0, s>>>(a);
   QCU_CHECK_LAUNCH();
 }
 void launch_bxout(int kind, const BatchArgs &a, cudaStream_t s) {
-  if (kind == SOA64) kb_xout<SOA64><<<persistent_grid(a, BB), BB, 0, s>>>(a);
-  else kb_xout<SOA32><<<persistent_grid(a, BB), BB, 0, s>>>(a);
+  if (kind == SOA64) kb_xout<SOA64><<<persistent_grid(a, kb_xout<SOA64>), BB, 0, s>>>(a);
+  else kb_xout<SOA32><<<persistent_grid(a, kb_xout<SOA32>), BB, 0, s>>>(a);
   QCU_CHECK_LAUNCH();
 }
 void launch_bloop_cond(const BatchArgs &a, cudaGraphConditionalHandle h, unsigned cap, cudaStream_t s) {
@@ -675,15 +687,15 @@ void launch_bloop_cond(const BatchArgs &a, cudaGraphConditionalHandle h, unsigne
   QCU_CHECK_LAUNCH();
 }
 void launch_bgcr_multidot(const BatchArgs &a, int k, cudaStream_t s) {
-  kb_gcr_multidot<<<persistent_grid(a, BB), BB, 0, s>>>(a, k);
+  kb_gcr_multidot<<<tile_grid(a), BB, 0, s>>>(a, k);
   QCU_CHECK_LAUNCH();
 }
 void launch_bgcr_orth(const BatchArgs &a, int k, cudaStream_t s) {
-  kb_gcr_orth<<<persistent_grid(a, BB), BB, 0, s>>>(a, k);
+  kb_gcr_orth<<<tile_grid(a), BB, 0, s>>>(a, k);
   QCU_CHECK_LAUNCH();
 }
 void launch_bgcr_update(const BatchArgs &a, int k, cudaStream_t s) {
-  kb_gcr_update<<<persistent_grid(a, BB), BB, 0, s>>>(a, k);
+  kb_gcr_update<<<tile_grid(a), BB, 0, s>>>(a, k);
   QCU_CHECK_LAUNCH();
 }
 

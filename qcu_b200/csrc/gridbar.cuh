@@ -15,7 +15,7 @@
 
 namespace qcu {
 
-constexpr int GRID_RED_BLOCKS = 256;  // at most
+constexpr int GRID_RED_BLOCKS = 148 * 3;  // at most
 constexpr int GRID_RED_VALUES = 8;    // sums of one reduction, at most
 struct GridRed {
   unsigned count;  // arrivals
@@ -29,6 +29,30 @@ struct GridRedShared {
   double in[32][GRID_RED_VALUES];
   int ok;
 };
+
+// one thread of a block counts it in and waits until the counter has reached target
+__device__ __forceinline__ int grid_arrive_wait(GridRed *g, unsigned target) {
+  __threadfence();
+  atomicAdd(&g->count, 1u);
+  unsigned c, polls = 0;
+  do {
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&g->count) : "memory");
+    if (++polls >= GRID_RED_POLLS) {
+      atomicExch(&g->failed, 1);
+      return 0;
+    }
+  } while ((int)(c - target) < 0);
+  __threadfence();
+  return 1;
+}
+
+// grid_allreduce without sums: a barrier (it takes an epoch like one)
+__device__ __forceinline__ bool grid_barrier(GridRed *g, unsigned base, unsigned epoch, GridRedShared &sh) {
+  __syncthreads();
+  if (threadIdx.x == 0) sh.ok = grid_arrive_wait(g, base + epoch * gridDim.x);
+  __syncthreads();
+  return sh.ok != 0;
+}
 
 // The sums over the grid of v[0..N) of the threads of every `step`-th warp of
 // each block (the others' are not looked at), into tot (shared memory, N
@@ -58,32 +82,23 @@ __device__ __forceinline__ bool grid_allreduce(GridRed *g, unsigned base, unsign
       __stcg(&g->part[epoch & 1][lane][blockIdx.x], q);
     }
     __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      atomicAdd(&g->count, 1u);
-      const unsigned target = base + epoch * gridDim.x;
-      unsigned c, polls = 0;
-      int ok = 1;
-      do {
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(&g->count) : "memory");
-        if (++polls >= GRID_RED_POLLS) {
-          atomicExch(&g->failed, 1);
-          ok = 0;
-          break;
-        }
-      } while ((int)(c - target) < 0);
-      __threadfence();
-      sh.ok = ok;
-    }
+    if (lane == 0) sh.ok = grid_arrive_wait(g, base + epoch * gridDim.x);
   }
   __syncthreads();
   if (!sh.ok) return false;
-  for (int k = warp; k < N; k += nw) {
-    double q = 0.0;
-    for (int i = lane; i < gridDim.x; i += 32) q += __ldcg(&g->part[epoch & 1][k][i]);
-    q = warp_sum(q);
-    if (lane == 0) tot[k] = q;
+  double q[N];  // value k by warp k % nw; a warp's loads and sums side by side
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    q[k] = 0.0;
+    if (k % nw == warp)
+      for (int i = lane; i < gridDim.x; i += 32) q[k] += __ldcg(&g->part[epoch & 1][k][i]);
   }
+#pragma unroll
+  for (int k = 0; k < N; k++)
+    if (k % nw == warp) {
+      q[k] = warp_sum(q[k]);
+      if (lane == 0) tot[k] = q[k];
+    }
   __syncthreads();
   return true;
 }

@@ -96,6 +96,7 @@ struct Spinor {
 // ---------------------------------------------------------------- per-device context
 // Streams, the solver state block and the reduction partials persist across
 // API calls (one context per device, created on first use).
+struct GridRed;
 struct Context {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -110,6 +111,7 @@ struct Context {
   DevBuf *legacy_clover = nullptr;
   DevBuf *legacy_bad = nullptr;
   DevBuf *legacy_gauge = nullptr;
+  GridRed *grid_red = nullptr;  // device; the state of cooperative kernels' reductions
   std::mutex mu;
   void ensure_partials(size_t blocks);
 };
@@ -183,6 +185,25 @@ void launch_xrupdate(int kind, int Vh, const VecSet &vs, Context &ctx, int gate,
 void launch_xfold(int kind, int Vh, const VecSet &vs, SolverState *st, int gate, cudaStream_t s);
 void launch_rconv(int kind, int Vh, const VecSet &vs, Context &ctx, int gate, cudaStream_t s);
 void launch_init(int kind, int Vh, const VecSet &vs, Context &ctx, cudaStream_t s);
+// The GCR's inner solve (16-bit spinors and links) on M_pc z = r64 from zero as
+// one cooperative kernel (inner_small.cu): vs's inner vectors and x as scratch,
+// z (SOA64) the result, st->iter, rr and status what it did.  c0, c1: CSOA32
+// inverse clover of the even and odd sites, or null.
+struct InnerArgs {
+  Geom g;
+  VecSet vs;
+  void *tmp = nullptr, *p2 = nullptr;  // 16-bit scratch beside vs (p2: p's second buffer)
+  float *tmpn = nullptr, *p2n = nullptr;
+  void *z = nullptr;
+  const void *gauge = nullptr, *c0 = nullptr, *c1 = nullptr;
+  double k2 = 0.0, t_bc = 1.0, rel2 = 0.0;
+  int maxiter = 0;
+  SolverState *st = nullptr;
+  GridRed *red = nullptr;
+};
+constexpr int INNER_SMALL_VH = 3 * 148 * 32;  // three 32-site tiles an SM: where the graph of kernels overtakes it
+bool inner_small_fits(int Vh);
+void launch_inner_small(const InnerArgs &a, int sms, cudaStream_t s);
 // device-side loop condition for a graph WHILE node: continue while !st->done (at most cap passes)
 void launch_loop_cond(SolverState *st, cudaGraphConditionalHandle h, unsigned cap, cudaStream_t s);
 void launch_convert(int kin, int kout, int Vh, const void *in, const float *in_n, void *out, float *out_n,

@@ -24,6 +24,7 @@
 // nu_post MR steps.  The FP64 true residual decides convergence.
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <memory>
 #include <vector>
 
@@ -413,9 +414,9 @@ __global__ void __launch_bounds__(32 * CAPPLY_WARPS) k_mg_capply(MGGeom m, const
 }
 
 struct CState {
-  GridRed red;
   int status;          // of the last solve
   long long total_it;  // iterations summed over the solves since the last reset
+  GridRed red;         // its partials, at the end, stay on the device
 };
 struct CoarseArgs {
   MGGeom m;
@@ -910,7 +911,7 @@ void coarse_solve(MG &mg, Context &ctx) {
 // the state of the coarse solves since the last reset, on the host; throws if a barrier gave up
 CState coarse_state(MG &mg, cudaStream_t st) {
   CState cs;
-  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, sizeof(CState), cudaMemcpyDeviceToHost, st));
+  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, offsetof(CState, red) + offsetof(GridRed, part), cudaMemcpyDeviceToHost, st));
   QCU_CUDA(cudaStreamSynchronize(st));
   if (cs.red.failed) {
     QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, sizeof(CState), st));

@@ -4,6 +4,7 @@
 #include <map>
 #include <memory>
 
+#include "gridbar.cuh"
 #include "internal.h"
 
 namespace qcu {
@@ -163,6 +164,8 @@ Context &context() {
   QCU_CUDA(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev));
   QCU_CUDA(cudaMalloc(&c->st, sizeof(SolverState)));
   QCU_CUDA(cudaMemset(c->st, 0, sizeof(SolverState)));
+  QCU_CUDA(cudaMalloc(&c->grid_red, sizeof(GridRed)));
+  QCU_CUDA(cudaMemset(c->grid_red, 0, sizeof(GridRed)));
   QCU_CUDA(cudaMallocHost(&c->st_host, sizeof(SolverState)));
   memset(c->st_host, 0, sizeof(SolverState));
   c->ensure_partials(MAX_REDUCE_BLOCKS);

@@ -13,6 +13,7 @@
 #include <cstring>
 
 #include "gcr.h"
+#include "gridbar.cuh"
 #include "nn.h"
 #include "solver.h"
 #include "mg.h"
@@ -334,6 +335,7 @@ static cudaGraphExec_t capture_inner_solve_while(Dsl &dP, Workspace &w, const Ve
 namespace {
 struct GcrSpace {
   Spinor W[GCR_MAXK], Z[GCR_MAXK], znew, wnew, zin;
+  Spinor p2;  // 16-bit scratch of the small lattices' inner solve
   void prepare(int m, int Vh) {
     for (int j = 0; j < m; j++) {
       W[j].alloc(SOA64, Vh);
@@ -380,7 +382,29 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
   long long nodes = 0;  // 0: device-side WHILE loop (launches counted from the iteration count)
   long long per_iter = 8;  // kernels per pass of the WHILE body (measured at capture)
   cudaGraphExec_t inner = nullptr;
-  if (pc != 1) {
+  // 16-bit inner solves of small lattices: one cooperative kernel instead of a graph
+  const bool small = pc != 1 && dP.kind == SOA16 && inner_small_fits(Vh);
+  InnerArgs ia;
+  if (small) {
+    ia.g = dP.G.g;
+    ia.vs = vin;
+    ia.tmp = w.tmp.data.p;
+    ia.tmpn = w.tmp.norm.as<float>();
+    gs.p2.alloc(SOA16, Vh);
+    ia.p2 = gs.p2.data.p;
+    ia.p2n = gs.p2.norm.as<float>();
+    ia.z = gs.zin.data.p;
+    ia.gauge = dP.G.g16.p;
+    ia.c0 = clov ? dP.G.Ainv32[0].p : nullptr;
+    ia.c1 = clov ? dP.G.Ainv32[1].p : nullptr;
+    ia.k2 = k2;
+    ia.t_bc = dP.G.t_bc;
+    ia.rel2 = init.inner_rel2;
+    ia.maxiter = prm.inner_iters;
+    ia.st = ctx.st;
+    ia.red = ctx.grid_red;
+  }
+  if (pc != 1 && !small) {
     try {
       inner = capture_inner_solve_while(dP, w, vin, kappa, clov, prm.inner_iters, gs.zin, per_iter);
     } catch (const Error &) {
@@ -442,7 +466,9 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
           d64(1, w.tmp64, w.aux, clov, -k2, &gs.znew, 1.0);
           mg_minres_scale(*prm.mg, ctx, gs.znew.data.p, w.aux.data.p, w.r64.data.p);
         }
-        if (pc != 1) {
+        if (small) {
+          launch_inner_small(ia, ctx.sms, st);
+        } else if (pc != 1) {
           QCU_CUDA(cudaGraphLaunch(inner, st));
           if (nodes) note_launch(nodes);
         }
@@ -461,11 +487,11 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
             a.beta[2 * j + 1] = S.sums[2 * j + 1] / nw[j];
           }
           info.iterations += pc == 1 ? 1 : S.iter;  // inner iterations of this step
-          if (pc != 1 && !nodes) note_launch(2 + per_iter * std::max(S.iter, 1));
+          if (inner && !nodes) note_launch(2 + per_iter * std::max(S.iter, 1));
         } else {
           const int it = pc == 1 ? 1 : read_state(ctx).iter;
           info.iterations += it;
-          if (pc != 1 && !nodes) note_launch(2 + per_iter * std::max(it, 1));
+          if (inner && !nodes) note_launch(2 + per_iter * std::max(it, 1));
         }
         launch_gcr_orth(Vh, a, ctx, st);
         SolverState S = read_state(ctx);
@@ -490,6 +516,15 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
     throw;
   }
   if (inner) cudaGraphExecDestroy(inner);
+  if (small) {  // a wait of the kernel's barriers that gave up
+    int failed = 0;
+    QCU_CUDA(cudaMemcpyAsync(&failed, &ctx.grid_red->failed, sizeof(int), cudaMemcpyDeviceToHost, st));
+    QCU_CUDA(cudaStreamSynchronize(st));
+    if (failed) {
+      QCU_CUDA(cudaMemsetAsync(ctx.grid_red, 0, sizeof(GridRed), st));
+      throw Error(2, "solve: a barrier of the inner solve timed out");
+    }
+  }
   if (pc == 3) mg_check_coarse(*prm.mg, ctx);
   if (info.status == ST_RUNNING && info.iterations >= prm.maxiter) info.status = ST_MAXITER;
 }

@@ -477,3 +477,24 @@ def test_dslashQcu_on_partial_warps(q, latt, shift):
         ref = O.dslash(psi[1 - p], U, latt, p)
         assert rel(host(dst[shift:shift + n]).reshape(ref.shape), ref) <= 1e-13
         assert bool(torch.isnan(dst[n if shift == 0 else 0].real))
+
+
+@pytest.mark.parametrize("latt", [[2, 2, 2, 2], [6, 2, 2, 6], [10, 2, 6, 4], [12, 8, 12, 12]])
+@pytest.mark.parametrize("clover", [False, True])
+def test_gcr_inner_solve_on_small_lattices(q, latt, clover):
+    """The one-kernel inner solve: fewer sites than a tile of 32 (8), a partial last tile (72, 240) and more tiles than
+    blocks (6912 sites, 216 tiles), Wilson and clover; the true residual by the oracle's operator."""
+    U = O.gauge_smooth(latt, 0.25, 31)
+    b = O.fermion_gauss(O.full_shape(latt), 32)
+    kappa, c = 0.12, 0.12 if clover else 0.0
+    A = [O.clover_build(U, latt, p, c) for p in (0, 1)] if clover else [None, None]
+    x, y = empty_like_dev(O.full_shape(latt)), empty_like_dev(O.full_shape(latt))
+    kw = dict(tol=1e-11, maxiter=4000, solver="gcr", precision=16, inner_iters=40, inner_tol=0.05, gcr_k=4, clover=clover)
+    with q.Gauge(dev(U), latt, t_boundary=-1.0, clover_coeff=c) as G:
+        info = G.invert(x, dev(b), kappa, **kw)
+        G.invert(y, dev(b), kappa, **kw)
+        assert np.array_equal(host(x), host(y))
+        short = G.invert(y, dev(b), kappa, **dict(kw, inner_iters=1))  # the inner iteration cap
+    assert info["status"] == 1 and info["fallback"] == 0 and short["status"] == 1
+    r = b - O.mfull(host(x), U, latt, kappa, -1.0, True, A[0], A[1])
+    assert np.linalg.norm(r) <= 1.05e-11 * np.linalg.norm(b)

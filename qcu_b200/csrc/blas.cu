@@ -65,10 +65,13 @@ __global__ void __launch_bounds__(BLAS_BLOCK) k_supdate(int Vh, VecSet vs, Solve
 // x += alpha p + omega s ; r = s - omega t ; reduce <rt, r>, |r|^2  -> FIN_XR
 template <int K, int XK>
 __global__ void __launch_bounds__(BLAS_BLOCK) k_xrupdate(int Vh, VecSet vs, SolverState *st, double *partials,
-                                                          int gate) {
+                                                          int gate, LoopCond lc) {
   using T = Real<K>;
   using TX = Real<XK>;
-  if (!gate_open(st, gate)) return;
+  if (!gate_open(st, gate)) {  // nothing to do: end the loop
+    if (blockIdx.x == 0 && threadIdx.x == 0) set_loop_cond(lc, st);
+    return;
+  }
   const Cpx<T> a((T)st->alpha[0], (T)st->alpha[1]), w((T)st->omega[0], (T)st->omega[1]);
   const Cpx<TX> ax((TX)st->alpha[0], (TX)st->alpha[1]), wx((TX)st->omega[0], (TX)st->omega[1]);
   double red[3] = {0, 0, 0};
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(BLAS_BLOCK) k_xrupdate(int Vh, VecSet vs, Solv
     site_dot<T>(rt, q, red[0], red[1]);
     site_norm2<T>(q, red[2]);
   }
-  grid_reduce<3, BLAS_BLOCK>(red, RedCtx{st, partials, FIN_XR});
+  grid_reduce<3, BLAS_BLOCK>(red, RedCtx{st, partials, FIN_XR, lc});
 }
 
 // x64 += x ; x = 0
@@ -257,27 +260,7 @@ __global__ void __launch_bounds__(BLAS_BLOCK) k_dots(int Vh, void *a, float *an,
   grid_reduce<4, BLAS_BLOCK>(red, RedCtx{st, partials, FIN_STORE});
 }
 
-// Condition of a device-side WHILE loop over solver iterations (a CUDA graph
-// conditional node): continue while the solver is not done.  The guard
-// bounds the loop whatever happens to `done`: after `cap` passes it stops
-// and reports the solve as having hit its iteration limit.
-__global__ void k_loop_cond(SolverState *st, cudaGraphConditionalHandle h, unsigned cap) {
-  const unsigned n = ++st->loop_guard;
-  bool go = st->done == 0;
-  if (go && n >= cap) {
-    st->status = ST_MAXITER;
-    st->done = 1;
-    go = false;
-  }
-  cudaGraphSetConditional(h, go ? 1u : 0u);
-}
-
 // ---------------------------------------------------------------- launchers
-void launch_loop_cond(SolverState *st, cudaGraphConditionalHandle h, unsigned cap, cudaStream_t s) {
-  k_loop_cond<<<1, 1, 0, s>>>(st, h, cap);
-  QCU_CHECK_LAUNCH();
-}
-
 #define QCU_DISPATCH_K(kind, F, ...)                   \
   switch (kind) {                                      \
     case SOA64: F<SOA64> __VA_ARGS__; break;           \
@@ -294,13 +277,13 @@ void launch_supdate(int kind, int Vh, const VecSet &vs, SolverState *st, int gat
   QCU_DISPATCH_K(kind, k_supdate, <<<blas_grid(Vh), BLAS_BLOCK, 0, s>>>(Vh, vs, st, gate));
   QCU_CHECK_LAUNCH();
 }
-void launch_xrupdate(int kind, int Vh, const VecSet &vs, Context &ctx, int gate, cudaStream_t s) {
+void launch_xrupdate(int kind, int Vh, const VecSet &vs, Context &ctx, int gate, cudaStream_t s, const LoopCond &lc) {
   const int g = blas_grid(Vh);
   ctx.ensure_partials(g);
   switch (kind) {
-    case SOA64: k_xrupdate<SOA64, SOA64><<<g, BLAS_BLOCK, 0, s>>>(Vh, vs, ctx.st, ctx.partials, gate); break;
-    case SOA32: k_xrupdate<SOA32, SOA32><<<g, BLAS_BLOCK, 0, s>>>(Vh, vs, ctx.st, ctx.partials, gate); break;
-    case SOA16: k_xrupdate<SOA16, SOA32><<<g, BLAS_BLOCK, 0, s>>>(Vh, vs, ctx.st, ctx.partials, gate); break;
+    case SOA64: k_xrupdate<SOA64, SOA64><<<g, BLAS_BLOCK, 0, s>>>(Vh, vs, ctx.st, ctx.partials, gate, lc); break;
+    case SOA32: k_xrupdate<SOA32, SOA32><<<g, BLAS_BLOCK, 0, s>>>(Vh, vs, ctx.st, ctx.partials, gate, lc); break;
+    case SOA16: k_xrupdate<SOA16, SOA32><<<g, BLAS_BLOCK, 0, s>>>(Vh, vs, ctx.st, ctx.partials, gate, lc); break;
     default: throw Error(1, "unsupported spinor kind");
   }
   QCU_CHECK_LAUNCH();

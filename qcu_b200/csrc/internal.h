@@ -181,7 +181,8 @@ struct VecSet {
 };
 void launch_pupdate(int kind, int Vh, const VecSet &vs, SolverState *st, int gate, cudaStream_t s);
 void launch_supdate(int kind, int Vh, const VecSet &vs, SolverState *st, int gate, cudaStream_t s);
-void launch_xrupdate(int kind, int Vh, const VecSet &vs, Context &ctx, int gate, cudaStream_t s);
+void launch_xrupdate(int kind, int Vh, const VecSet &vs, Context &ctx, int gate, cudaStream_t s,
+                     const LoopCond &lc = LoopCond());
 void launch_xfold(int kind, int Vh, const VecSet &vs, SolverState *st, int gate, cudaStream_t s);
 void launch_rconv(int kind, int Vh, const VecSet &vs, Context &ctx, int gate, cudaStream_t s);
 void launch_init(int kind, int Vh, const VecSet &vs, Context &ctx, cudaStream_t s);
@@ -204,8 +205,6 @@ struct InnerArgs {
 constexpr int INNER_SMALL_VH = 3 * 148 * 32;  // three 32-site tiles an SM: where the graph of kernels overtakes it
 bool inner_small_fits(int Vh);
 void launch_inner_small(const InnerArgs &a, int sms, cudaStream_t s);
-// device-side loop condition for a graph WHILE node: continue while !st->done (at most cap passes)
-void launch_loop_cond(SolverState *st, cudaGraphConditionalHandle h, unsigned cap, cudaStream_t s);
 void launch_convert(int kin, int kout, int Vh, const void *in, const float *in_n, void *out, float *out_n,
                     cudaStream_t s);
 void launch_axpby(int kind, int Vh, double a, void *x, float *xn, double b, void *y, float *yn, cudaStream_t s);

@@ -31,13 +31,14 @@ struct SolverState {
 };
 
 // gate modes: which kernels of a captured iteration actually run
-enum Gate { GATE_ALWAYS = 0, GATE_NOT_DONE = 1, GATE_UPDATE = 2 };
+enum Gate { GATE_ALWAYS = 0, GATE_NOT_DONE = 1, GATE_UPDATE = 2, GATE_STEP = 3 };  // STEP: not done, and no reliable update due
 
 __device__ __forceinline__ bool gate_open(const SolverState *st, int gate) {
   if (gate == GATE_ALWAYS || st == nullptr) return true;
   volatile const SolverState *v = st;
   if (gate == GATE_NOT_DONE) return v->done == 0;
-  return v->update != 0 && v->done == 0;
+  if (gate == GATE_STEP) return (v->done | v->update) == 0;  // both loads at once: one round trip per block
+  return (v->update != 0) & (v->done == 0);
 }
 
 enum FinOp {
@@ -194,10 +195,22 @@ __device__ __forceinline__ void site_norm2(const Cpx<T> a[12], double &n2) {
   }
 }
 
+// The WHILE node of a captured iteration loop, whose condition the finalize of
+// an iteration's last reduction sets (no kernel is launched for it): another
+// pass while the solve is not done and no reliable update is due.
+struct LoopCond {
+  cudaGraphConditionalHandle handle = 0;
+  int on = 0;
+};
+__device__ __forceinline__ void set_loop_cond(const LoopCond &lc, const SolverState *st) {
+  if (lc.on) cudaGraphSetConditional(lc.handle, st->done || st->update ? 0u : 1u);
+}
+
 struct RedCtx {
   SolverState *st;
   double *partials;  // value-major: value k of block b at [k * gridDim.x + b] (room for RED_MAXV values)
   int op;
+  LoopCond lc;
 };
 
 
@@ -271,6 +284,7 @@ __device__ __forceinline__ void grid_reduce(double v[NV], const RedCtx &rc) {
 #pragma unroll
     for (int k = 0; k < RED_MAXV; k++) s[k] = k < NV ? tot[k] : 0.0;
     finalize(rc.st, rc.op, s);
+    set_loop_cond(rc.lc, rc.st);
     rc.st->ticket = 0;
     __threadfence();
   }

@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <vector>
 
 #include "gcr.h"
 #include "gridbar.cuh"
@@ -207,23 +208,113 @@ double finish_solution(Dsl &d64, double kappa, bool clov, Spinor &be, Spinor &bo
   return rr;
 }
 
-// one BiCGSTAB iteration (plus the gated reliable-update sequence)
-static void enqueue_iteration(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, double kappa, bool clov) {
+// one BiCGSTAB iteration; gate: when it runs (GATE_NOT_DONE where no reliable
+// update can be due: a load less per block); lc: the captured loop whose
+// condition its end sets
+static void enqueue_step(Dsl &dP, Workspace &w, const VecSet &vs, double kappa, bool clov, int gate,
+                         const LoopCond &lc = LoopCond()) {
   Context &ctx = dP.ctx;
   const int Vh = dP.G.g.Vh, kind = dP.kind;
   const double k2 = kappa * kappa;
-  launch_pupdate(kind, Vh, vs, ctx.st, GATE_NOT_DONE, ctx.stream);
-  dP(0, w.p, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_NOT_DONE);
-  dP(1, w.tmp, w.v, clov, -k2, &w.p, 1.0, nullptr, 0, RED_DOT_RT, FIN_ALPHA, &w.rt, GATE_NOT_DONE);
-  launch_supdate(kind, Vh, vs, ctx.st, GATE_NOT_DONE, ctx.stream);
-  dP(0, w.s, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_NOT_DONE);
-  dP(1, w.tmp, w.t, clov, -k2, &w.s, 1.0, nullptr, 0, RED_TS_TT, FIN_OMEGA, nullptr, GATE_NOT_DONE);
-  launch_xrupdate(kind, Vh, vs, ctx, GATE_NOT_DONE, ctx.stream);
-  // reliable update: x64 += x; r64 = b' - M_pc x64 (FP64); r = r64
+  launch_pupdate(kind, Vh, vs, ctx.st, gate, ctx.stream);
+  dP(0, w.p, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, gate);
+  dP(1, w.tmp, w.v, clov, -k2, &w.p, 1.0, nullptr, 0, RED_DOT_RT, FIN_ALPHA, &w.rt, gate);
+  launch_supdate(kind, Vh, vs, ctx.st, gate, ctx.stream);
+  dP(0, w.s, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, gate);
+  dP(1, w.tmp, w.t, clov, -k2, &w.s, 1.0, nullptr, 0, RED_TS_TT, FIN_OMEGA, nullptr, gate);
+  launch_xrupdate(kind, Vh, vs, ctx, gate, ctx.stream, lc);
+}
+// the gated reliable update: x64 += x; r64 = b' - M_pc x64 (FP64); r = r64
+static void enqueue_update(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, double kappa, bool clov) {
+  Context &ctx = dP.ctx;
+  const int Vh = dP.G.g.Vh;
   launch_xfold(w.x.kind, Vh, vs, ctx.st, GATE_UPDATE, ctx.stream);
   d64(0, w.x64, w.tmp64, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_UPDATE);
-  d64(1, w.tmp64, w.r64, clov, k2, &w.bp, 1.0, &w.x64, -1.0, RED_NORM, FIN_RTRUE, nullptr, GATE_UPDATE);
-  launch_rconv(kind, Vh, vs, ctx, GATE_UPDATE, ctx.stream);
+  d64(1, w.tmp64, w.r64, clov, kappa * kappa, &w.bp, 1.0, &w.x64, -1.0, RED_NORM, FIN_RTRUE, nullptr, GATE_UPDATE);
+  launch_rconv(dP.kind, Vh, vs, ctx, GATE_UPDATE, ctx.stream);
+}
+static void enqueue_iteration(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, double kappa, bool clov) {
+  enqueue_step(dP, w, vs, kappa, clov, GATE_NOT_DONE);
+  enqueue_update(dP, d64, w, vs, kappa, clov);
+}
+
+// ends whatever capture a failure left open on the stream, and drops the graph
+static void abandon_capture(cudaStream_t st, cudaGraph_t g) {
+  cudaStreamCaptureStatus cs;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
+    cudaGraph_t junk;
+    cudaStreamEndCapture(st, &junk);
+  }
+  cudaGetLastError();
+  if (g) cudaGraphDestroy(g);
+}
+static cudaGraph_t add_conditional(cudaGraph_t g, cudaGraphConditionalNodeType type, cudaGraphConditionalHandle h,
+                                   const cudaGraphNode_t *after, cudaGraphNode_t *node) {
+  cudaGraphNodeParams cp = {};
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = h;
+  cp.conditional.type = type;
+  cp.conditional.size = 1;
+  QCU_CUDA(cudaGraphAddNode(node, g, after, after ? 1 : 0, &cp));
+  return cp.conditional.phGraph_out[0];
+}
+// the node of a captured chain that nothing depends on
+static cudaGraphNode_t last_node(cudaGraph_t g) {
+  size_t n = 0;
+  QCU_CUDA(cudaGraphGetNodes(g, nullptr, &n));
+  std::vector<cudaGraphNode_t> nodes(n);
+  QCU_CUDA(cudaGraphGetNodes(g, nodes.data(), &n));
+  for (cudaGraphNode_t nd : nodes) {
+    size_t out = 0;
+    QCU_CUDA(cudaGraphNodeGetDependentNodes(nd, nullptr, &out));
+    if (out == 0) return nd;
+  }
+  throw Error(3, "solver graph: no last node");
+}
+
+// One iteration as the body of a WHILE node of graph g (after `after`, or
+// first).  The iteration's x and r update sets the node's condition, from the
+// new state, or to "stop" when it finds nothing to do, so every pass counts an
+// iteration towards the limit or ends the loop.  (Four iterations a pass save
+// less between passes than the gated ones after the last cost: a 24^3 x 48 GCR
+// solve 19.2 -> 19.8 ms, 16^3 x 32 FP64 BiCGSTAB 10.53 -> 10.59 ms.)
+static cudaGraphNode_t add_step_loop(cudaGraph_t g, const cudaGraphNode_t *after, Dsl &dP, Workspace &w, const VecSet &vs,
+                                     double kappa, bool clov, int gate, long long &per_pass) {
+  cudaStream_t st = dP.ctx.stream;
+  LoopCond lc;
+  QCU_CUDA(cudaGraphConditionalHandleCreate(&lc.handle, g, 1, cudaGraphCondAssignDefault));
+  lc.on = 1;
+  cudaGraphNode_t loop;
+  cudaGraph_t body = add_conditional(g, cudaGraphCondTypeWhile, lc.handle, after, &loop);
+  QCU_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+  const long long before = launch_count();
+  enqueue_step(dP, w, vs, kappa, clov, gate, lc);
+  per_pass = launch_count() - before;
+  QCU_CUDA(cudaStreamEndCapture(st, &body));
+  return loop;
+}
+// The BiCGSTAB loop, up to its end or the next reliable update, as a graph.  (A
+// graph of 8 to 32 unrolled iterations takes as long to instantiate as several
+// of them to run on a small lattice, and launches four gated kernels an
+// iteration for an update that comes once in dozens.)
+static cudaGraphExec_t capture_bicgstab(Dsl &dP, Workspace &w, const VecSet &vs, double kappa, bool clov,
+                                        long long &per_pass) {
+  cudaStream_t st = dP.ctx.stream;
+  const long long before = launch_count();
+  cudaGraph_t g = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  try {
+    QCU_CUDA(cudaGraphCreate(&g, 0));
+    add_step_loop(g, nullptr, dP, w, vs, kappa, clov, GATE_STEP, per_pass);
+    QCU_CUDA(cudaGraphInstantiate(&exec, g, 0));
+  } catch (...) {
+    abandon_capture(st, g);
+    set_launch_count(before);
+    throw;
+  }
+  cudaGraphDestroy(g);
+  set_launch_count(before);  // counted from the iterations once they have run
+  return exec;
 }
 
 // Inner preconditioner solve of the GCR outer loop: BiCGSTAB in the inner
@@ -242,15 +333,7 @@ static cudaGraphExec_t capture_inner_solve(Dsl &dP, Workspace &w, const VecSet &
   QCU_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   try {
     launch_init(kind, Vh, vs, ctx, st);
-    for (int k = 0; k < iters; k++) {
-      launch_pupdate(kind, Vh, vs, ctx.st, GATE_NOT_DONE, st);
-      dP(0, w.p, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_NOT_DONE);
-      dP(1, w.tmp, w.v, clov, -k2, &w.p, 1.0, nullptr, 0, RED_DOT_RT, FIN_ALPHA, &w.rt, GATE_NOT_DONE);
-      launch_supdate(kind, Vh, vs, ctx.st, GATE_NOT_DONE, st);
-      dP(0, w.s, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_NOT_DONE);
-      dP(1, w.tmp, w.t, clov, -k2, &w.s, 1.0, nullptr, 0, RED_TS_TT, FIN_OMEGA, nullptr, GATE_NOT_DONE);
-      launch_xrupdate(kind, Vh, vs, ctx, GATE_NOT_DONE, st);
-    }
+    for (int k = 0; k < iters; k++) enqueue_step(dP, w, vs, kappa, clov, GATE_NOT_DONE);
     launch_convert(w.x.kind, SOA64, Vh, w.x.data.p, w.x.norm.as<float>(), z_out.data.p, nullptr, st);
   } catch (...) {
     cudaStreamEndCapture(st, &graph);
@@ -267,63 +350,34 @@ static cudaGraphExec_t capture_inner_solve(Dsl &dP, Workspace &w, const VecSet &
 
 // The same inner solve as a graph with a conditional WHILE node: init, then
 // the iteration body repeated on the device until the solver state says done
-// (converged, breakdown, or inner_iters reached; a guard counter bounds the
-// loop in any case), then the conversion.  No empty launches after
+// (converged, breakdown, or inner_iters reached), then the conversion.  The x
+// and r update that ends an iteration sets the condition: from the new state,
+// or to "stop" when it finds the solve over, so every pass counts an iteration
+// towards inner_iters or ends the loop.  No empty launches after
 // convergence and no host involvement.  `iters_out` is not known at capture
 // time: the caller reads st->iter after each replay.
 static cudaGraphExec_t capture_inner_solve_while(Dsl &dP, Workspace &w, const VecSet &vs, double kappa, bool clov,
-                                                 int iters, Spinor &z_out, long long &per_iter) {
+                                                 Spinor &z_out, long long &per_pass) {
   Context &ctx = dP.ctx;
   const int Vh = dP.G.g.Vh, kind = dP.kind;
-  const double k2 = kappa * kappa;
   cudaStream_t st = ctx.stream;
   const auto mode = cudaStreamCaptureModeThreadLocal;
   const long long before = launch_count();
   cudaGraph_t g = nullptr;
-  QCU_CUDA(cudaGraphCreate(&g, 0));
   cudaGraphExec_t exec = nullptr;
   try {
+    QCU_CUDA(cudaGraphCreate(&g, 0));
     QCU_CUDA(cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, mode));
     launch_init(kind, Vh, vs, ctx, st);
     QCU_CUDA(cudaStreamEndCapture(st, &g));
-    cudaGraphNode_t init_node;
-    size_t n = 1;
-    QCU_CUDA(cudaGraphGetNodes(g, &init_node, &n));
-    require(n == 1, "inner solve graph: unexpected init capture");
-    cudaGraphConditionalHandle h;
-    QCU_CUDA(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t loop;
-    QCU_CUDA(cudaGraphAddNode(&loop, g, &init_node, 1, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    QCU_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, mode));
-    const long long body0 = launch_count();
-    launch_pupdate(kind, Vh, vs, ctx.st, GATE_NOT_DONE, st);
-    dP(0, w.p, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_NOT_DONE);
-    dP(1, w.tmp, w.v, clov, -k2, &w.p, 1.0, nullptr, 0, RED_DOT_RT, FIN_ALPHA, &w.rt, GATE_NOT_DONE);
-    launch_supdate(kind, Vh, vs, ctx.st, GATE_NOT_DONE, st);
-    dP(0, w.s, w.tmp, clov, 1.0, nullptr, 0, nullptr, 0, RED_NONE, FIN_STORE, nullptr, GATE_NOT_DONE);
-    dP(1, w.tmp, w.t, clov, -k2, &w.s, 1.0, nullptr, 0, RED_TS_TT, FIN_OMEGA, nullptr, GATE_NOT_DONE);
-    launch_xrupdate(kind, Vh, vs, ctx, GATE_NOT_DONE, st);
-    launch_loop_cond(ctx.st, h, (unsigned)iters + 2u, st);
-    per_iter = launch_count() - body0;  // kernels per pass of the loop body
-    QCU_CUDA(cudaStreamEndCapture(st, &body));
+    const cudaGraphNode_t init_node = last_node(g);
+    const cudaGraphNode_t loop = add_step_loop(g, &init_node, dP, w, vs, kappa, clov, GATE_NOT_DONE, per_pass);
     QCU_CUDA(cudaStreamBeginCaptureToGraph(st, g, &loop, nullptr, 1, mode));
     launch_convert(w.x.kind, SOA64, Vh, w.x.data.p, w.x.norm.as<float>(), z_out.data.p, nullptr, st);
     QCU_CUDA(cudaStreamEndCapture(st, &g));
     QCU_CUDA(cudaGraphInstantiate(&exec, g, 0));
   } catch (...) {
-    cudaStreamCaptureStatus cs;
-    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
-      cudaGraph_t junk;
-      cudaStreamEndCapture(st, &junk);
-    }
-    cudaGetLastError();
-    cudaGraphDestroy(g);
+    abandon_capture(st, g);
     set_launch_count(before);
     throw;
   }
@@ -380,7 +434,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
   VecSet vin = vs;
   vin.r64 = pc >= 2 ? w.aux.data.p : w.r64.data.p;
   long long nodes = 0;  // 0: device-side WHILE loop (launches counted from the iteration count)
-  long long per_iter = 8;  // kernels per pass of the WHILE body (measured at capture)
+  long long per_pass = 0;  // kernels per pass of the WHILE body
   cudaGraphExec_t inner = nullptr;
   // 16-bit inner solves of small lattices: one cooperative kernel instead of a graph
   const bool small = pc != 1 && dP.kind == SOA16 && inner_small_fits(Vh);
@@ -406,7 +460,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
   }
   if (pc != 1 && !small) {
     try {
-      inner = capture_inner_solve_while(dP, w, vin, kappa, clov, prm.inner_iters, gs.zin, per_iter);
+      inner = capture_inner_solve_while(dP, w, vin, kappa, clov, gs.zin, per_pass);
     } catch (const Error &) {
       // conditional graph nodes unavailable: fixed-length capture with gated iterations
       inner = capture_inner_solve(dP, w, vin, kappa, clov, prm.inner_iters, gs.zin, nodes);
@@ -487,11 +541,11 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
             a.beta[2 * j + 1] = S.sums[2 * j + 1] / nw[j];
           }
           info.iterations += pc == 1 ? 1 : S.iter;  // inner iterations of this step
-          if (inner && !nodes) note_launch(2 + per_iter * std::max(S.iter, 1));
+          if (inner && !nodes) note_launch(2 + per_pass * std::max(S.iter, 1));
         } else {
           const int it = pc == 1 ? 1 : read_state(ctx).iter;
           info.iterations += it;
-          if (inner && !nodes) note_launch(2 + per_iter * std::max(it, 1));
+          if (inner && !nodes) note_launch(2 + per_pass * std::max(it, 1));
         }
         launch_gcr_orth(Vh, a, ctx, st);
         SolverState S = read_state(ctx);
@@ -554,7 +608,32 @@ static SolverState run_bicgstab(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &v
   if (!S.done) {
     cudaGraphExec_t exec = nullptr;
     long long nodes = 0;
-    if (use_graph) {
+    if (use_graph && prm.chunk == 0) {
+      long long per_pass = 0;
+      try {
+        exec = capture_bicgstab(dP, w, vs, kappa, clov, per_pass);
+      } catch (const Error &) {
+        exec = nullptr;  // conditional graph nodes unavailable: unrolled graphs of `chunk` iterations
+      }
+      if (exec) {
+        try {
+          while (!S.done) {  // every turn advances st->iter, and the iteration that reaches maxiter sets done
+            const int it0 = S.iter;
+            QCU_CUDA(cudaGraphLaunch(exec, st));
+            enqueue_update(dP, d64, w, vs, kappa, clov);
+            S = read_state(ctx);
+            require(S.done || S.iter > it0, "solver made no progress (internal error)");
+            note_launch(per_pass * std::max(S.iter - it0, 1));
+          }
+        } catch (...) {
+          cudaGraphExecDestroy(exec);
+          throw;
+        }
+        cudaGraphExecDestroy(exec);
+        exec = nullptr;
+      }
+    }
+    if (!S.done && use_graph) {
       cudaGraph_t graph;
       const long long before = launch_count();
       QCU_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -575,7 +654,7 @@ static SolverState run_bicgstab(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &v
     // passes; the cap below only guards against a logic error
     const long long max_passes = (long long)maxiter / chunk + 8;
     try {
-      for (long long pass = 0;; pass++) {
+      for (long long pass = 0; !S.done; pass++) {
         require(pass < max_passes, "solver did not terminate within maxiter (internal error)");
         if (exec) {
           QCU_CUDA(cudaGraphLaunch(exec, st));
@@ -584,7 +663,6 @@ static SolverState run_bicgstab(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &v
           for (int k = 0; k < chunk; k++) enqueue_iteration(dP, d64, w, vs, kappa, clov);
         }
         S = read_state(ctx);
-        if (S.done) break;
       }
     } catch (...) {
       if (exec) cudaGraphExecDestroy(exec);

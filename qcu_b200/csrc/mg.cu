@@ -173,8 +173,26 @@ struct FineVec {
 };
 __device__ __forceinline__ size_t hidx(int s, int comp) { return blk_base<12>(s) + (size_t)comp * SB; }
 
-// coarse c[B][ch nvec + k] = <v_k^ch, r>_B: per k a warp sum, then one pass
-// over the warps
+// The sums over the warp of 16 values, value lane / 2 in each lane: a halving
+// exchange, 16 shuffles where a butterfly per value takes 80.
+__device__ __forceinline__ double warp_sum16(double (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int w = 8, off = 16; w >= 1; w >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (i < w) {
+        const double send = up ? v[i] : v[i + w], keep = up ? v[i + w] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// coarse c[B][ch nvec + k] = <v_k^ch, r>_B: warp sums for four vectors at a
+// time, then one pass over the warps.  Bound by the near-null vectors' bytes
+// (96 n_vec a site): 16^3 x 32, n_vec 12: 77 -> 46 us.
 __global__ void __launch_bounds__(MG_MAXBLOCK) k_mg_restrict(MGGeom m, const float2 *nv, FineVec r, float2 *cv) {
   __shared__ double red[MG_MAXBLOCK / 32][MG_MAXVEC][4];
   const int B = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5, nw = blockDim.x >> 5;
@@ -183,24 +201,25 @@ __global__ void __launch_bounds__(MG_MAXBLOCK) k_mg_restrict(MGGeom m, const flo
   double2 rv[12];
 #pragma unroll
   for (int comp = 0; comp < 12; comp++) rv[comp] = rp ? rp[hidx(c.s, comp)] : make_double2(0, 0);
-  for (int k = 0; k < m.nvec; k++) {
-    double v[4] = {0, 0, 0, 0};
-    if (rp) {
+  for (int k0 = 0; k0 < m.nvec; k0 += 4) {
+    double v[16];
 #pragma unroll
-      for (int comp = 0; comp < 12; comp++) {
-        const int ch = comp / 6;
-        const float2 a = nv[nidx(m, k, B, t, comp)];
-        v[2 * ch] += (double)a.x * rv[comp].x + (double)a.y * rv[comp].y;
-        v[2 * ch + 1] += (double)a.x * rv[comp].y - (double)a.y * rv[comp].x;
+    for (int i = 0; i < 16; i++) v[i] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (rp && k0 + q < m.nvec) {
+        const float2 *p = nv + nidx(m, k0 + q, B, t, 0);
+#pragma unroll
+        for (int comp = 0; comp < 12; comp++) {
+          const int i = 4 * q + 2 * (comp / 6);
+          const float2 a = p[comp * m.bsites];
+          v[i] += (double)a.x * rv[comp].x + (double)a.y * rv[comp].y;
+          v[i + 1] += (double)a.x * rv[comp].y - (double)a.y * rv[comp].x;
+        }
       }
     }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-    if (lane == 0)
-#pragma unroll
-      for (int i = 0; i < 4; i++) red[w][k][i] = v[i];
+    const double tot = warp_sum16(v);
+    if (!(lane & 1) && k0 + (lane >> 3) < m.nvec) red[w][k0 + (lane >> 3)][(lane >> 1) & 3] = tot;
   }
   __syncthreads();
   for (int i = t; i < 2 * m.nvec; i += blockDim.x) {  // i = ch nvec + k
@@ -674,7 +693,31 @@ __global__ void __launch_bounds__(MG_RED) k_mg_dots(int64_t n, const V *a, const
   if (threadIdx.x == 0)
     for (int k = 0; k < 3; k++) part[blockIdx.x * 3 + k] = v[k];
 }
-// x += a y; r -= a w (the MR and GCR updates in one pass)
+// the same onto the solver state's sums (in block order, no host in between)
+__global__ void __launch_bounds__(MG_RED) k_mg_dots_dev(int64_t n, const double2 *a, const double2 *b, SolverState *st,
+                                                       double *partials) {
+  double v[3] = {0, 0, 0};
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double2 x = a[i], y = b[i];
+    v[0] += x.x * y.x + x.y * y.y;
+    v[1] += x.x * y.y - x.y * y.x;
+    v[2] += x.x * x.x + x.y * x.y;
+  }
+  grid_reduce<3, MG_RED>(v, RedCtx{st, partials, FIN_STORE});
+}
+// an MR step with its multiple from the sums <q, s>, |q|^2: x += a s; s -= a q
+// (nothing when q = 0, as s is then)
+__global__ void k_mg_mr(int64_t n, double2 *x, double2 *s, const double2 *q, const SolverState *st) {
+  const double qq = st->sums[2];
+  if (!(qq > 0)) return;
+  const double2 a = make_double2(st->sums[0] / qq, st->sums[1] / qq);
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double2 ss = s[i], ww = q[i], xx = x[i];
+    x[i] = make_double2(xx.x + a.x * ss.x - a.y * ss.y, xx.y + a.x * ss.y + a.y * ss.x);
+    s[i] = make_double2(ss.x - a.x * ww.x + a.y * ww.y, ss.y - a.x * ww.y - a.y * ww.x);
+  }
+}
+// x += a y; r -= a w (the GCR update in one pass)
 __global__ void k_mg_axpy2(int64_t n, double2 *x, const double2 *y, double2 *r, const double2 *w, double2 a) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 yy = y[i], ww = w[i], xx = x[i], rr = r[i];
@@ -821,8 +864,12 @@ void lin3(cudaStream_t st, int64_t n, V *out, C a, const V *x, C b = C(0, 0), co
   QCU_CHECK_LAUNCH();
 }
 
-// out = M in on full FP64 vectors: out_p = A_p in_p - kappa D_{p <- 1-p} in_{1-p}
-void mat(MG &mg, Context &ctx, const double2 *in, double2 *out) {
+// out = M in on full FP64 vectors: out_p = A_p in_p - kappa D_{p <- 1-p} in_{1-p};
+// dots: also <out, in> and |out|^2 in the solver state's sums[0..2] (from the
+// two hops themselves without a clover term, whose epilogue holds both vectors:
+// 16^3 x 32, an MR step 62 us without a word to the host; dots of their own took
+// 59 us of kernels and the round trip between them)
+void mat(MG &mg, Context &ctx, const double2 *in, double2 *out, bool dots = false) {
   const GaugeHandle &G = *mg.G;
   const size_t half = (size_t)mg.m.Vp * 12;
   for (int p = 0; p < 2; p++) {
@@ -839,8 +886,16 @@ void mat(MG &mg, Context &ctx, const double2 *in, double2 *out) {
       d.x1 = mg.tmp.p;
     } else {
       d.x1 = in + p * half;
+      if (dots) {
+        d.red = RED_TS_TT;
+        d.fin = p ? FIN_ADD : FIN_STORE;
+      }
     }
     launch_dslash(SOA64, GSOA64, CSOA64, G.g, d, ctx, ctx.stream);
+  }
+  if (dots && G.has_clover) {
+    k_mg_dots_dev<<<mg_grid(mg.nfull()), MG_RED, 0, ctx.stream>>>(mg.nfull(), out, in, ctx.st, ctx.partials);
+    QCU_CHECK_LAUNCH();
   }
 }
 
@@ -938,11 +993,9 @@ void smooth(MG &mg, Context &ctx, const double2 *r, double2 *e, int steps, bool 
     residual(mg, ctx, e, r, s);
   }
   for (int k = 0; k < steps; k++) {
-    mat(mg, ctx, s, q);
-    double d[3];
-    dots(mg, st, n, q, s, d);  // <M s, s>, |M s|^2
-    if (!(d[2] > 0)) break;
-    axpy2(st, n, e, s, s, q, C(d[0] / d[2], d[1] / d[2]));
+    mat(mg, ctx, s, q, true);  // with <M s, s>, |M s|^2
+    k_mg_mr<<<mg_grid(n), MG_RED, 0, st>>>(n, e, s, q, ctx.st);
+    QCU_CHECK_LAUNCH();
   }
 }
 

@@ -43,6 +43,7 @@ __device__ __forceinline__ bool gate_open(const SolverState *st, int gate) {
 
 enum FinOp {
   FIN_STORE = 0,  // sums -> st->sums
+  FIN_ADD,        // st->sums += sums
   FIN_ALPHA,      // alpha = rho / <rt, v>
   FIN_OMEGA,      // omega = <t, s> / <t, t>
   FIN_XR,         // rho_prev = rho; rho = <rt, r>; rr = |r|^2; iteration bookkeeping
@@ -57,6 +58,9 @@ __device__ inline void finalize(SolverState *st, int op, const double *s) {
   switch (op) {
     case FIN_STORE:
       for (int k = 0; k < RED_MAXV; k++) st->sums[k] = s[k];
+      break;
+    case FIN_ADD:
+      for (int k = 0; k < RED_MAXV; k++) st->sums[k] += s[k];
       break;
     case FIN_ALPHA: {
       Cpx<double> den(s[0], s[1]);

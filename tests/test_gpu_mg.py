@@ -120,3 +120,23 @@ def test_gcr_with_coarse_grid_correction(q, clover):
         with pytest.raises(q.QcuError):
             G.invert(x, dev(b), kappa, tol=1e-10, solver="gcr", clover=clover, precond=3)
         mg.close()
+
+
+@pytest.mark.parametrize("n_vec,block", [(1, [4, 4, 4, 4]), (6, [2, 4, 4, 4]), (16, [4, 4, 4, 4]), (5, [8, 4, 4, 4])])
+def test_multigrid_shapes_of_the_coarse_kernels(q, n_vec, block):
+    """The coarse solve's kernel at 1 to 16 vectors (2 to 32 rows) and 16 to 64 aggregates, and the restriction's groups
+    of four vectors with 1, 2 and 0 left over: P^dag P = 1, the Galerkin identity, and a solve by the oracle's operator."""
+    latt, kappa = [8, 8, 8, 8], 0.12
+    U = O.gauge_smooth(latt, 0.25, 51)
+    b = O.fermion_gauss(O.full_shape(latt), 52)
+    x = empty_like_dev(O.full_shape(latt))
+    with q.Gauge(dev(U), latt, t_boundary=-1.0) as G:
+        mg = q.Multigrid(G, kappa, geo_block_size=block, n_vec=n_vec, setup_maxiter=16, coarse_tol=0.05,
+                         coarse_maxiter=50)
+        orth, gal = mg.check()
+        info = mg.invert(x, dev(b), tol=1e-10, maxiter=300)
+        mg.close()
+    assert orth <= 1e-5 and gal <= 1e-5
+    assert info["status"] == 1
+    r = b - O.mfull(host(x), U, latt, kappa, -1.0)
+    assert np.linalg.norm(r) <= 1.05e-10 * np.linalg.norm(b)

@@ -156,6 +156,10 @@ enum RedKind { RED_NONE = 0, RED_DOT_RT = 1, RED_TS_TT = 2, RED_NORM = 3 };
 void launch_dslash(int kind, int gkind, int ckind, const Geom &g, const DslashArgs &a, Context &ctx,
                    cudaStream_t s);
 
+// the same for FP32 / 16-bit spinors with the result in PyQuda's layout (out:
+// complex128; no epilogue sources, no reduction)
+void launch_dslash_out(int kind, int gkind, const Geom &g, const DslashArgs &a, cudaStream_t s);
+
 // out(par) = D in on PyQuda-layout half spinors and links (hop_records.cu); in
 // and out must not overlap
 void launch_hop_records(const Geom &g, const void *in, void *out, const void *gauge, int par, double t_bc,

@@ -804,16 +804,29 @@ void handle_dslash(GaugeHandle &G, void *out, const void *in, int par, int use_c
     return;
   }
   Workspace &w = workspace();
-  w.aux.alloc(SOA64, Vh);
-  w.tmp64.alloc(SOA64, Vh);
-  w.r.alloc(kind, Vh);
-  w.tmp.alloc(kind, Vh);
-  Spinor &a = kind == SOA64 ? w.aux : w.r, &b = kind == SOA64 ? w.tmp64 : w.tmp;
   QCU_CUDA(cudaDeviceSynchronize());
-  Dsl d{G, ctx, kind, links16 ? GSOA16 : -1};
-  launch_convert(AOS64, kind, Vh, in, nullptr, a.data.p, a.norm.as<float>(), ctx.stream);
-  d(par, a, b, use_clover != 0, 1.0);
-  launch_convert(kind, AOS64, Vh, b.data.p, b.norm.as<float>(), out, nullptr, ctx.stream);
+  if (kind == SOA64) {  // overlapping buffers
+    w.aux.alloc(SOA64, Vh);
+    w.tmp64.alloc(SOA64, Vh);
+    Dsl d{G, ctx, SOA64};
+    launch_convert(AOS64, SOA64, Vh, in, nullptr, w.aux.data.p, nullptr, ctx.stream);
+    d(par, w.aux, w.tmp64, use_clover != 0, 1.0);
+    launch_convert(SOA64, AOS64, Vh, w.tmp64.data.p, nullptr, out, nullptr, ctx.stream);
+  } else {
+    w.r.alloc(kind, Vh);
+    launch_convert(AOS64, kind, Vh, in, nullptr, w.r.data.p, w.r.norm.as<float>(), ctx.stream);
+    DslashArgs d;
+    d.in = w.r.data.p;
+    d.in_norm = w.r.norm.as<float>();
+    d.out = out;
+    const int gk = links16 ? GSOA16 : gkind_of(kind);
+    d.gauge = gk == GSOA32 ? G.g32.p : G.g16.p;
+    d.clover = use_clover ? G.Ainv32[par].p : nullptr;
+    d.parity = par;
+    d.t_bc = G.t_bc;
+    d.a = 1.0;
+    launch_dslash_out(kind, gk, G.g, d, ctx.stream);
+  }
   QCU_CUDA(cudaStreamSynchronize(ctx.stream));
 }
 

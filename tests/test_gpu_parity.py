@@ -498,3 +498,29 @@ def test_gcr_inner_solve_on_small_lattices(q, latt, clover):
     assert info["status"] == 1 and info["fallback"] == 0 and short["status"] == 1
     r = b - O.mfull(host(x), U, latt, kappa, -1.0, True, A[0], A[1])
     assert np.linalg.norm(r) <= 1.05e-11 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("prec", [32, 16, 3216])
+@pytest.mark.parametrize("clover", [False, True])
+def test_reduced_precision_hop_writes_the_callers_buffer(q, prec, clover):
+    """240 sites per parity (a partial block and warp): aligned to 32 and to 16 bytes only and in place of the input,
+    the same bits each time and within the storage's bar of the oracle; nothing written beside."""
+    import torch
+
+    latt, c = [10, 2, 6, 4], 0.11 if clover else 0.0
+    U, psi = _fields(latt, "smooth", 27)
+    n = psi[1].size
+    expect = O.dslash(psi[1], U, latt, 0, -1.0)
+    if clover:
+        expect = O.clover_apply(O.clover_invert(O.clover_build(U, latt, 0, c)), expect)
+    got = []
+    with q.Gauge(dev(U), latt, t_boundary=-1.0, clover_coeff=c) as G:
+        for start, to in ((0, n + 24), (0, n + 25), (0, 0), (1, 0)):
+            buf = torch.full((2 * n + 60,), float("nan"), dtype=torch.complex128, device="cuda")
+            buf[start:start + n] = dev(psi[1]).reshape(-1)
+            out = buf[start + to:start + to + n]
+            G.dslash(out, buf[start:start + n], 0, clover=clover, precision=prec)
+            got.append(host(out))
+            assert bool(torch.isnan(buf[start + to + n:].real).all())
+    assert all(np.array_equal(g, got[0]) for g in got)
+    assert rel(got[0].reshape(expect.shape), expect) <= (1e-6 if prec == 32 else 2e-4)

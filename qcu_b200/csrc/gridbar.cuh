@@ -15,7 +15,7 @@
 
 namespace qcu {
 
-constexpr int GRID_RED_BLOCKS = 148 * 3;  // at most
+constexpr int GRID_RED_BLOCKS = 148 * 4;  // at most
 constexpr int GRID_RED_VALUES = 8;    // sums of one reduction, at most
 struct GridRed {
   unsigned count;  // arrivals

@@ -415,6 +415,29 @@ __device__ __forceinline__ float2 mg_row(const float4 *Yb, int nc, const float2 
   return make_float2(re0 + re1, im0 + im1);
 }
 
+// the same from global memory with C loads of a lane in flight at a time: 7, as
+// a warp of eight has 13 or 14 column pairs of 24 rows (14 at a time cost the
+// registers of a quarter of the blocks)
+template <int C>
+__device__ __forceinline__ float2 mg_row_wide(const float4 *Yb, int nc, const float2 *xin, int jp0, int jp1) {
+  float re0 = 0.f, im0 = 0.f, re1 = 0.f, im1 = 0.f;
+  for (int jp = jp0; jp < jp1; jp += C) {
+    float4 a[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) a[c] = jp + c < jp1 ? __ldg(Yb + (size_t)(jp + c) * nc) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      if (jp + c >= jp1) break;
+      const float2 x0 = xin[2 * (jp + c)], x1 = xin[2 * (jp + c) + 1];
+      re0 = fmaf(a[c].x, x0.x, fmaf(-a[c].y, x0.y, re0));
+      im0 = fmaf(a[c].x, x0.y, fmaf(a[c].y, x0.x, im0));
+      re1 = fmaf(a[c].z, x1.x, fmaf(-a[c].w, x1.y, re1));
+      im1 = fmaf(a[c].z, x1.y, fmaf(a[c].w, x1.x, im1));
+    }
+  }
+  return make_float2(re0 + re1, im0 + im1);
+}
+
 // out = A_c in, one warp per aggregate, lane = row; the neighbours' inputs
 // staged in shared memory (the set-up check; the solve is k_mg_coarse)
 __global__ void __launch_bounds__(32 * CAPPLY_WARPS) k_mg_capply(MGGeom m, const float4 *Y, const float2 *in,
@@ -459,23 +482,33 @@ struct CoarseArgs {
 //   <rt, r> = <rt, s> - omega <rt, t>,   |r|^2 = |s|^2 - |<t, s>|^2 / |t|^2.
 // The 32 warps of a block share the columns of 1, 2 or 4 aggregates (lane =
 // row).  Bound by the latency of its barriers and of A_c's entries from L2
-// (from HBM where A_c is larger; where every block's part fits, it stays in
-// shared memory).  16^3 x 32, 4^4 aggregates, 24 rows: 12.8 us an iteration, 4.3
-// of them the barriers, where nine kernels an iteration took 49 us.
+// (where every block's part fits, it stays in shared memory).  16^3 x 32, 4^4
+// aggregates, 24 rows: 12.8 us an iteration, 4.3 of them the barriers, where
+// nine kernels an iteration took 49 us.
+// A_c larger than MGC_STREAM is read from HBM, and the chain from an aggregate's
+// neighbours to its inputs to its product has to be covered: four blocks of 256
+// threads an SM, each with an aggregate of its own at its own place in the chain,
+// and the next aggregate's matrix asked for ahead.  32^3 x 64 (340 MB): 165 us an
+// iteration, against 226 with one block of 1024 (211 with four blocks but nothing
+// asked for ahead) and 181 with nine kernels; 24^3 x 48 (108 MB): 70, 89 and 91.
 constexpr int MGC_THREADS = 1024;
+// below it the one large block is as fast (24^4, 54 MB: 35 us against 37; 16^2 x
+// 24 x 32: 27 against 30), as the matrices stay in L2
+constexpr size_t MGC_STREAM = (size_t)64 << 20;
 constexpr int MGC_SMEM = 180 * 1024;  // the most a block's matrices may take of its shared memory
-template <bool CACHED>
-__global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
+template <bool CACHED, int T>
+__global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) {
+  constexpr bool STREAM = T < MGC_THREADS;
   extern __shared__ float4 ysm[];  // CACHED: the entries of the block's aggregates
-  __shared__ float2 xin[4][9 * 2 * MG_MAXVEC];
-  __shared__ float2 psum[MGC_THREADS / 32][32];
-  __shared__ int nb[4][9];
+  __shared__ float2 xin[T / 256][9 * 2 * MG_MAXVEC];
+  __shared__ float2 psum[T / 32][32];
+  __shared__ int nb[T / 256][9];
   __shared__ GridRedShared red;
   __shared__ double tot[8];
   __shared__ double2 sc[5];  // alpha, omega, beta, beta omega, rho
   __shared__ int done;
   const int nc = a.m.nc, J = 9 * nc, P = J / 2;
-  const int tpa = MGC_THREADS / a.apb, wpa = tpa / 32;
+  const int tpa = T / a.apb, wpa = tpa / 32;
   const int al = threadIdx.x / tpa, lt = threadIdx.x % tpa, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = blockIdx.x * a.apb, stride = gridDim.x * a.apb;
   const int jp0 = (lt >> 5) * P / wpa, jp1 = ((lt >> 5) + 1) * P / wpa;
@@ -489,6 +522,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
     __syncthreads();
     if (mine && lane < nc)
       psum[warp][lane] = CACHED ? mg_row<true>(ysm + (size_t)al * P * nc + lane, nc, xin[al], jp0, jp1)
+                       : STREAM ? mg_row_wide<7>(a.Y + (size_t)B * P * nc + lane, nc, xin[al], jp0, jp1)
                                 : mg_row<false>(a.Y + (size_t)B * P * nc + lane, nc, xin[al], jp0, jp1);
     __syncthreads();
     float2 o = make_float2(0.f, 0.f);
@@ -498,6 +532,13 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
   };
   auto neighbours = [&](int B) {
     if (B < a.m.nblocks && lt < 9) nb[al][lt] = mg_cnbr(a.m, B, lt);
+  };
+  // STREAM: has the matrix of the aggregate after B (of the next application,
+  // after the last) fetched into L2 while B's inputs are formed and used
+  auto prefetch = [&](int B) {
+    const int Bn = B + stride < a.m.nblocks ? B + stride : first + al;
+    if (STREAM && lt == 32 && Bn < a.m.nblocks)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.Y + (size_t)Bn * P * nc), "r"(P * nc * 16) : "memory");
   };
 
   double v1[1] = {0.0}, v2[2], v8[8];
@@ -511,7 +552,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
   }
   if constexpr (CACHED) {
     const int n = min(a.apb, a.m.nblocks - first) * P * nc;
-    for (int i = threadIdx.x; i < n; i += MGC_THREADS) ysm[i] = __ldg(a.Y + (size_t)first * P * nc + i);
+    for (int i = threadIdx.x; i < n; i += T) ysm[i] = __ldg(a.Y + (size_t)first * P * nc + i);
     neighbours(first + al);
   }
   bool ok = grid_allreduce<1>(&a.st->red, count0, ++epoch, v1, wpa, tot, red);
@@ -536,6 +577,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
       if constexpr (!CACHED) {
         __syncthreads();
         neighbours(B);
+        prefetch(B);
         __syncthreads();
       }
       auto stage = [&](int i, int d, int row) {
@@ -591,6 +633,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) k_mg_coarse(CoarseArgs a) {
       if constexpr (!CACHED) {
         __syncthreads();
         neighbours(B);
+        prefetch(B);
         __syncthreads();
       }
       auto stage = [&](int i, int d, int row) {
@@ -950,16 +993,21 @@ void coarse_solve(MG &mg, Context &ctx) {
   a.st = mg.cstate.as<CState>();
   a.tol2 = mg.p.coarse_tol * mg.p.coarse_tol;
   a.maxit = mg.p.coarse_maxiter;
+  const size_t part = (size_t)(9 * a.m.nc / 2) * a.m.nc * sizeof(float4);  // of A_c, an aggregate's
+  const bool stream = part * mg.m.nblocks > MGC_STREAM;
+  const int T = stream ? 256 : MGC_THREADS, per = MGC_THREADS / T;
   // spread the aggregates over the SMs before a block takes several at a time
-  a.apb = mg.m.nblocks <= ctx.sms ? 1 : (mg.m.nblocks <= 2 * ctx.sms ? 2 : 4);
-  const int grid = std::min(std::min(ctx.sms, GRID_RED_BLOCKS), (mg.m.nblocks + a.apb - 1) / a.apb);
+  a.apb = stream || mg.m.nblocks <= ctx.sms ? 1 : (mg.m.nblocks <= 2 * ctx.sms ? 2 : 4);
+  const int grid = std::min(std::min(per * ctx.sms, GRID_RED_BLOCKS), (mg.m.nblocks + a.apb - 1) / a.apb);
   // A_c stays in shared memory where every block has one set of aggregates that fits
-  const size_t smem = (size_t)a.apb * (9 * a.m.nc / 2) * a.m.nc * sizeof(float4);
-  const bool cached = smem <= MGC_SMEM && (int64_t)grid * a.apb >= a.m.nblocks;
-  const void *k = cached ? reinterpret_cast<const void *>(k_mg_coarse<true>) : reinterpret_cast<const void *>(k_mg_coarse<false>);
+  const size_t smem = a.apb * part;
+  const bool cached = !stream && smem <= MGC_SMEM && (int64_t)grid * a.apb >= a.m.nblocks;
+  const void *k = stream   ? reinterpret_cast<const void *>(k_mg_coarse<false, 256>)
+                  : cached ? reinterpret_cast<const void *>(k_mg_coarse<true, MGC_THREADS>)
+                           : reinterpret_cast<const void *>(k_mg_coarse<false, MGC_THREADS>);
   if (cached) QCU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MGC_SMEM));
   void *args[] = {&a};
-  QCU_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(MGC_THREADS), args, cached ? smem : 0, ctx.stream));
+  QCU_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(T), args, cached ? smem : 0, ctx.stream));
   note_launch(1);
 }
 

@@ -140,3 +140,25 @@ def test_multigrid_shapes_of_the_coarse_kernels(q, n_vec, block):
     assert info["status"] == 1
     r = b - O.mfull(host(x), U, latt, kappa, -1.0)
     assert np.linalg.norm(r) <= 1.05e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n_vec,latt,block", [(16, [16, 16, 16, 16], [2, 2, 4, 4]), (11, [16, 16, 16, 32], [2, 2, 4, 4])])
+def test_multigrid_coarse_operator_larger_than_the_cache(q, n_vec, latt, block):
+    """A coarse operator above 64 MiB (four blocks an SM, the matrices asked for ahead; 32 and 22 rows, the last turn of
+    the blocks not full): the solve by the oracle's operator, and fewer outer steps than with one coarse iteration."""
+    kappa = 0.124
+    U = O.gauge_smooth(latt, 0.25, 61)
+    b = O.fermion_gauss(O.full_shape(latt), 62)
+    x = empty_like_dev(O.full_shape(latt))
+    outer = {}
+    with q.Gauge(dev(U), latt, t_boundary=-1.0) as G:
+        for cm in (1, 50):
+            mg = q.Multigrid(G, kappa, geo_block_size=block, n_vec=n_vec, setup_maxiter=32, coarse_tol=0.05,
+                             coarse_maxiter=cm)
+            info = mg.invert(x, dev(b), tol=1e-10, maxiter=300)
+            mg.close()
+            assert info["status"] == 1
+            outer[cm] = info["outer"]
+    assert outer[50] < outer[1], outer
+    r = b - O.mfull(host(x), U, latt, kappa, -1.0)
+    assert np.linalg.norm(r) <= 1.05e-10 * np.linalg.norm(b)

@@ -10,7 +10,16 @@
 // loads a turn, costs several us more.
 // The counter goes on rising from launch to launch (modulo 2^32): nothing has
 // to be reset, and launches of different sizes may follow one another.
+//
+// After a wait that gave up the counter says nothing any more, so `failed` stays
+// set and every later launch on the state returns at once (grid_red_failed); the
+// host looks at it with the next scalars it reads, ends the call with an error,
+// and clears the state where a call begins (grid_red_reset).
 #pragma once
+#include <cstddef>
+#include <cstdlib>
+#include <cstring>
+
 #include "reduce.cuh"
 
 namespace qcu {
@@ -20,7 +29,7 @@ constexpr int GRID_RED_VALUES = 8;    // sums of one reduction, at most
 struct GridRed {
   unsigned count;  // arrivals
   unsigned base;   // arrivals of the launches before
-  int failed;      // set when a wait gave up; the host reads and clears the state
+  int failed;      // set when a wait gave up
   double part[2][GRID_RED_VALUES][GRID_RED_BLOCKS];
 };
 constexpr unsigned GRID_RED_POLLS = 1u << 21;  // a second or two
@@ -44,6 +53,12 @@ __device__ __forceinline__ int grid_arrive_wait(GridRed *g, unsigned target) {
   } while ((int)(c - target) < 0);
   __threadfence();
   return 1;
+}
+
+// whether a wait of an earlier launch on this state gave up: then the kernel
+// returns before its first reduction (every thread of every block calls this)
+__device__ __forceinline__ bool grid_red_failed(const GridRed *g) {
+  return __syncthreads_or(*static_cast<const volatile int *>(&g->failed)) != 0;
 }
 
 // grid_allreduce without sums: a barrier (it takes an epoch like one)
@@ -106,6 +121,15 @@ __device__ __forceinline__ bool grid_allreduce(GridRed *g, unsigned base, unsign
 // by one thread of the grid, after its last reduction of the kernel
 __device__ __forceinline__ void grid_red_end(GridRed *g, unsigned base, unsigned epochs) {
   g->base = base + epochs * gridDim.x;
+}
+
+// host: a state as before its first launch, in stream order
+inline cudaError_t grid_red_reset(GridRed *g, cudaStream_t s) { return cudaMemsetAsync(g, 0, offsetof(GridRed, part), s); }
+// QCU_BARRIER_GIVE_UP = `name` ("inner" or "coarse") leaves the state as a wait that
+// gave up leaves it, before a launch: the host-side way the tests drive the error
+inline cudaError_t grid_red_inject(GridRed *g, const char *name, cudaStream_t s) {
+  const char *e = getenv("QCU_BARRIER_GIVE_UP");
+  return e && strcmp(e, name) == 0 ? cudaMemsetAsync(&g->failed, 1, sizeof(int), s) : cudaSuccess;
 }
 
 }  // namespace qcu

@@ -275,6 +275,10 @@ __global__ void __launch_bounds__(IS_THREADS, 1) k_inner_small(InnerArgs a) {
   __shared__ int state, next;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int Vh = a.g.Vh, ntile = (Vh + 31) / 32;
+  if (grid_red_failed(a.red)) {
+    if (threadIdx.x == 0) a.st->gave_up = 1;
+    return;
+  }
   const unsigned base = a.red->base;
   unsigned epoch = 0;
   const HopOfWarp hw = hop_of_warp(warp);
@@ -485,6 +489,10 @@ __global__ void __launch_bounds__(IS_THREADS, 1) k_inner_small(InnerArgs a) {
     }
   }
   __syncthreads();
+  if (!ok) {
+    if (threadIdx.x == 0) a.st->gave_up = 1;
+    return;
+  }
   // the result in FP64 (warp 2 and 3 own x)
   if (warp >= 2 && warp < 4)
     for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
@@ -516,6 +524,7 @@ void launch_inner_small(const InnerArgs &a, int sms, cudaStream_t s) {
   const void *k = a.c0 ? reinterpret_cast<const void *>(k_inner_small<true>) : reinterpret_cast<const void *>(k_inner_small<false>);
   InnerArgs arg = a;
   void *args[] = {&arg};
+  QCU_CUDA(grid_red_inject(a.red, "inner", s));
   QCU_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(IS_THREADS), args, 0, s));
   note_launch(1);
 }

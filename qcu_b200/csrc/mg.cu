@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(32 * CAPPLY_WARPS) k_mg_capply(MGGeom m, const
 }
 
 struct CState {
-  int status;          // of the last solve
+  int status;          // of the last solve that ended
   long long total_it;  // iterations summed over the solves since the last reset
   GridRed red;         // its partials, at the end, stay on the device
 };
@@ -511,6 +511,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
   const int tpa = T / a.apb, wpa = tpa / 32;
   const int al = threadIdx.x / tpa, lt = threadIdx.x % tpa, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = blockIdx.x * a.apb, stride = gridDim.x * a.apb;
+  if (grid_red_failed(&a.st->red)) return;
   const int jp0 = (lt >> 5) * P / wpa, jp1 = ((lt >> 5) + 1) * P / wpa;
   // the (at most two, as J <= 288 and tpa >= 256) inputs this thread stages: block d, row
   const int d0 = lt / nc, row0 = lt - d0 * nc, d1 = (lt + tpa) / nc, row1 = lt + tpa - d1 * nc;
@@ -556,13 +557,14 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
     neighbours(first + al);
   }
   bool ok = grid_allreduce<1>(&a.st->red, count0, ++epoch, v1, wpa, tot, red);
+  if (!ok) return;
   const double bb = tot[0];
-  int status = ok && bb > 0 ? ST_RUNNING : ST_CONVERGED, it = 0;
+  int status = bb > 0 ? ST_RUNNING : ST_CONVERGED, it = 0;
   if (threadIdx.x == 0) {
     sc[0] = sc[1] = sc[2] = sc[3] = make_double2(0, 0);
     sc[4] = make_double2(bb, 0.0);  // <rt, r> with rt = r = b
   }
-  for (; ok && status == ST_RUNNING; it++) {
+  for (; status == ST_RUNNING; it++) {
     const int cur = it & 1;
     float2 *rc = cur ? a.r1 : a.r0, *pc = cur ? a.p1 : a.p0, *vc = cur ? a.v1 : a.v0;
     const float2 *ro = cur ? a.r0 : a.r1, *po = cur ? a.p0 : a.p1, *vo = cur ? a.v0 : a.v1;
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
       }
     }
     ok = grid_allreduce<2>(&a.st->red, count0, ++epoch, v2, wpa, tot, red);
-    if (!ok) break;
+    if (!ok) return;
     const double2 rtv = make_double2(tot[0], tot[1]);
     if (!(rtv.x * rtv.x + rtv.y * rtv.y > 0)) {
       status = ST_BREAKDOWN;
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
       }
     }
     ok = grid_allreduce<8>(&a.st->red, count0, ++epoch, v8, wpa, tot, red);
-    if (!ok) break;
+    if (!ok) return;
     if (threadIdx.x == 0) {  // omega = 0 when t = 0 (then s = 0 too)
       const double it2 = tot[2] > 0 ? 1.0 / tot[2] : 0.0;
       const double2 w = make_double2(tot[0] * it2, tot[1] * it2);
@@ -721,9 +723,10 @@ __global__ void k_mg_lin3(int64_t n, V *out, double2 a, const V *x, double2 b, c
     out[i].y = im;
   }
 }
-// per-block partials of Re<a,b>, Im<a,b>, |a|^2 (<a,b> = sum conj(a) b)
+// per-block partials of Re<a,b>, Im<a,b>, |a|^2 (<a,b> = sum conj(a) b); behind
+// them, whether a barrier of the coarse solves so far gave up
 template <typename V>
-__global__ void __launch_bounds__(MG_RED) k_mg_dots(int64_t n, const V *a, const V *b, double *part) {
+__global__ void __launch_bounds__(MG_RED) k_mg_dots(int64_t n, const V *a, const V *b, const CState *cs, double *part) {
   __shared__ double sh[(MG_RED / 32) * 3];
   double v[3] = {0, 0, 0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -735,8 +738,9 @@ __global__ void __launch_bounds__(MG_RED) k_mg_dots(int64_t n, const V *a, const
   mg_block_sum<3>(v, sh);
   if (threadIdx.x == 0)
     for (int k = 0; k < 3; k++) part[blockIdx.x * 3 + k] = v[k];
+  if (blockIdx.x == 0 && threadIdx.x == 0) part[gridDim.x * 3] = cs->red.failed;
 }
-// the same onto the solver state's sums (in block order, no host in between)
+// the sums onto the solver state's sums (in block order, no host in between)
 __global__ void __launch_bounds__(MG_RED) k_mg_dots_dev(int64_t n, const double2 *a, const double2 *b, SolverState *st,
                                                        double *partials) {
   double v[3] = {0, 0, 0};
@@ -811,8 +815,10 @@ __global__ void k_mg_multiaxpy(int64_t n, double2 *out, Dirs W, int cnt) {
   }
 }
 
-// one parity (SOA64 half spinors, the Vh real sites only): block partials of <a, b>, |a|^2
-__global__ void __launch_bounds__(MG_RED) k_mg_half_dots(int Vh, const double2 *a, const double2 *b, double *part) {
+// one parity (SOA64 half spinors, the Vh real sites only): block partials of
+// <a, b>, |a|^2, and the same flag behind them
+__global__ void __launch_bounds__(MG_RED) k_mg_half_dots(int Vh, const double2 *a, const double2 *b, const CState *cs,
+                                                        double *part) {
   __shared__ double sh[(MG_RED / 32) * 3];
   double v[3] = {0, 0, 0};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)Vh * 12;
@@ -826,6 +832,7 @@ __global__ void __launch_bounds__(MG_RED) k_mg_half_dots(int Vh, const double2 *
   mg_block_sum<3>(v, sh);
   if (threadIdx.x == 0)
     for (int k = 0; k < 3; k++) part[blockIdx.x * 3 + k] = v[k];
+  if (blockIdx.x == 0 && threadIdx.x == 0) part[gridDim.x * 3] = cs->red.failed;
 }
 // z *= alpha; q = r - alpha q (one parity)
 __global__ void k_mg_half_mr(int Vh, double2 *z, double2 *q, const double2 *r, double2 al) {
@@ -887,16 +894,22 @@ FineVec slabs(const MG &mg, const double2 *v) {
   return FineVec{{p, p + (size_t)mg.m.Vp * 12}};
 }
 
-template <typename V>
-void dots(MG &mg, cudaStream_t st, int64_t n, const V *a, const V *b, double out[3]) {
-  const int gr = mg_grid(n);
-  k_mg_dots<V><<<gr, MG_RED, 0, st>>>(n, a, b, mg.part.as<double>());
-  QCU_CHECK_LAUNCH();
-  QCU_CUDA(cudaMemcpyAsync(mg.part_h.data(), mg.part.p, (size_t)gr * 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
+// the sums of gr blocks' three partials, on the host; throws when the flag
+// behind them says that a barrier gave up: nothing of the cycle is used then
+void read_sums(MG &mg, cudaStream_t st, int gr, double out[3]) {
+  QCU_CUDA(cudaMemcpyAsync(mg.part_h.data(), mg.part.p, ((size_t)gr * 3 + 1) * sizeof(double), cudaMemcpyDeviceToHost, st));
   QCU_CUDA(cudaStreamSynchronize(st));
+  if (mg.part_h[(size_t)gr * 3] != 0.0) throw Error(2, "mg: a barrier of the coarse solve timed out");
   out[0] = out[1] = out[2] = 0;
   for (int i = 0; i < gr; i++)
     for (int k = 0; k < 3; k++) out[k] += mg.part_h[(size_t)i * 3 + k];
+}
+template <typename V>
+void dots(MG &mg, cudaStream_t st, int64_t n, const V *a, const V *b, double out[3]) {
+  const int gr = mg_grid(n);
+  k_mg_dots<V><<<gr, MG_RED, 0, st>>>(n, a, b, mg.cstate.as<CState>(), mg.part.as<double>());
+  QCU_CHECK_LAUNCH();
+  read_sums(mg, st, gr, out);
 }
 
 template <typename V>
@@ -1007,20 +1020,19 @@ void coarse_solve(MG &mg, Context &ctx) {
                            : reinterpret_cast<const void *>(k_mg_coarse<false, MGC_THREADS>);
   if (cached) QCU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MGC_SMEM));
   void *args[] = {&a};
+  QCU_CUDA(grid_red_inject(&a.st->red, "coarse", ctx.stream));
   QCU_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(T), args, cached ? smem : 0, ctx.stream));
   note_launch(1);
 }
 
-// the state of the coarse solves since the last reset, on the host; throws if a barrier gave up
-CState coarse_state(MG &mg, cudaStream_t st) {
+constexpr size_t CSTATE_HEAD = offsetof(CState, red) + offsetof(GridRed, part);
+
+// the iterations of the coarse solves since the last reset, on the host
+long long coarse_iterations(MG &mg, cudaStream_t st) {
   CState cs;
-  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, offsetof(CState, red) + offsetof(GridRed, part), cudaMemcpyDeviceToHost, st));
+  QCU_CUDA(cudaMemcpyAsync(&cs, mg.cstate.p, CSTATE_HEAD, cudaMemcpyDeviceToHost, st));
   QCU_CUDA(cudaStreamSynchronize(st));
-  if (cs.red.failed) {
-    QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, sizeof(CState), st));
-    throw Error(2, "mg: a barrier of the coarse solve timed out");
-  }
-  return cs;
+  return cs.total_it;
 }
 
 void axpy2(cudaStream_t st, int64_t n, double2 *x, const double2 *y, double2 *r, const double2 *w, C a) {
@@ -1217,13 +1229,10 @@ double2 mg_minres_scale(MG &mg, Context &ctx, void *z, void *q, const void *r) {
   const int Vh = mg.m.Vh;
   const int gr = mg_grid((int64_t)Vh * 12);
   k_mg_half_dots<<<gr, MG_RED, 0, st>>>(Vh, static_cast<const double2 *>(q), static_cast<const double2 *>(r),
-                                        mg.part.as<double>());
+                                        mg.cstate.as<CState>(), mg.part.as<double>());
   QCU_CHECK_LAUNCH();
-  QCU_CUDA(cudaMemcpyAsync(mg.part_h.data(), mg.part.p, (size_t)gr * 3 * sizeof(double), cudaMemcpyDeviceToHost, st));
-  QCU_CUDA(cudaStreamSynchronize(st));
-  double d[3] = {0, 0, 0};
-  for (int i = 0; i < gr; i++)
-    for (int k = 0; k < 3; k++) d[k] += mg.part_h[(size_t)i * 3 + k];
+  double d[3];
+  read_sums(mg, st, gr, d);
   const double2 al = d[2] > 0 ? make_double2(d[0] / d[2], d[1] / d[2]) : make_double2(0, 0);
   k_mg_half_mr<<<gr, MG_RED, 0, st>>>(Vh, static_cast<double2 *>(z), static_cast<double2 *>(q),
                                       static_cast<const double2 *>(r), al);
@@ -1231,7 +1240,7 @@ double2 mg_minres_scale(MG &mg, Context &ctx, void *z, void *q, const void *r) {
   return al;
 }
 
-void mg_check_coarse(MG &mg, Context &ctx) { coarse_state(mg, ctx.stream); }
+void mg_reset_coarse(MG &mg, Context &ctx) { QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, CSTATE_HEAD, ctx.stream)); }
 
 double mg_setup_seconds(const MG &mg) { return mg.setup_seconds; }
 
@@ -1255,7 +1264,7 @@ MGInfo mg_solve(MG &mg, void *x_pyq, const void *b_pyq, double tol, int maxiter)
   QCU_CUDA(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double2), st));
   QCU_CUDA(cudaMemcpyAsync(r, b, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st));
   MGInfo info;
-  QCU_CUDA(cudaMemsetAsync(mg.cstate.p, 0, sizeof(CState), st));
+  mg_reset_coarse(mg, ctx);
   double d[3];
   dots(mg, st, n, b, b, d);
   const double bb = d[2];
@@ -1329,8 +1338,7 @@ MGInfo mg_solve(MG &mg, void *x_pyq, const void *b_pyq, double tol, int maxiter)
     rr = d[2];
   }
   info.true_residual = std::sqrt(rr / bb);
-  const CState cs = coarse_state(mg, st);
-  info.coarse_iters = (int)std::min<long long>(cs.total_it, 0x7fffffff);
+  info.coarse_iters = (int)std::min<long long>(coarse_iterations(mg, st), 0x7fffffff);
   for (int par = 0; par < 2; par++)
     launch_convert(SOA64, AOS64, Vh, x + par * half, nullptr, static_cast<char *>(x_pyq) + par * half_pyq, nullptr,
                    st);
@@ -1344,6 +1352,7 @@ void mg_check(MG &mg, double *orth_err, double *galerkin_err) {
   require(ctx.device == mg.device, "mg: the multigrid was set up on another device");
   std::lock_guard<std::mutex> lk(ctx.mu);
   cudaStream_t st = ctx.stream;
+  mg_reset_coarse(mg, ctx);
   const MGGeom &m = mg.m;
   const int64_t nc = mg.ncoarse();
   // a seeded coarse vector, uniform in [-1, 1) (xorshift64)

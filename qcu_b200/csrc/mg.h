@@ -46,11 +46,12 @@ double mg_setup_seconds(const MG &mg);
 // stream, the caller holds ctx.mu.
 void mg_coarse_odd(MG &mg, Context &ctx, const void *r_odd, void *z_odd);
 // with q = M_pc z on entry: alpha = <q, r> / |q|^2 (the minimal-residual
-// multiple of the correction), z *= alpha, q = r - alpha q; returns alpha
+// multiple of the correction), z *= alpha, q = r - alpha q; returns alpha;
+// throws when a barrier of the coarse solve before it gave up
 double2 mg_minres_scale(MG &mg, Context &ctx, void *z, void *q, const void *r);
 // throws unless mg was built on G for this kappa, with the clover term iff G has one
 void mg_require_compatible(const MG &mg, const GaugeHandle &G, double kappa, int use_clover);
-// throws if a barrier of a coarse solve gave up (waits for the stream)
-void mg_check_coarse(MG &mg, Context &ctx);
+// before the first coarse solve of a call: clears what an earlier call, ended by an error, may have left
+void mg_reset_coarse(MG &mg, Context &ctx);
 
 }  // namespace qcu

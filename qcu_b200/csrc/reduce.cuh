@@ -28,6 +28,7 @@ struct SolverState {
   int inner_mode;  // 1: a preconditioner solve (no reliable updates, stops on inner_rel2)
   unsigned ticket;
   unsigned loop_guard;  // body executions of a device-side WHILE loop since the last init
+  int gave_up;  // a grid barrier of k_inner_small gave up (set there, cleared by the host)
 };
 
 // gate modes: which kernels of a captured iteration actually run

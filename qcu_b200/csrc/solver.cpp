@@ -403,6 +403,11 @@ struct GcrSpace {
 GcrSpace &gcr_space() { return per_device<GcrSpace>(context()); }
 }  // namespace
 
+// the first thing read after an inner solve: its z is worth nothing when a barrier gave up
+static void require_inner(const SolverState &S) {
+  if (S.gave_up) throw Error(2, "solve: a barrier of the inner solve timed out");
+}
+
 // Flexible GCR(m) on M_pc in FP64 with the inner solve above as right
 // preconditioner: x64/r64 advance until the recursive |r|^2 <= tol2.
 static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const SolveParams &prm, double tol2,
@@ -430,7 +435,10 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
   require(pc == 0 || pc == 3 || prm.nn != nullptr, "solve: the network preconditioner needs a network");
   require(pc != 3 || prm.mg != nullptr, "solve: precond 3 needs a multigrid");
   if (pc == 1 || pc == 2) nn_prepare(*prm.nn, Vh);
-  if (pc == 3) mg_require_compatible(*prm.mg, dP.G, kappa, prm.use_clover);
+  if (pc == 3) {
+    mg_require_compatible(*prm.mg, dP.G, kappa, prm.use_clover);
+    mg_reset_coarse(*prm.mg, ctx);
+  }
   VecSet vin = vs;
   vin.r64 = pc >= 2 ? w.aux.data.p : w.r64.data.p;
   long long nodes = 0;  // 0: device-side WHILE loop (launches counted from the iteration count)
@@ -457,6 +465,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
     ia.maxiter = prm.inner_iters;
     ia.st = ctx.st;
     ia.red = ctx.grid_red;
+    QCU_CUDA(grid_red_reset(ctx.grid_red, st));
   }
   if (pc != 1 && !small) {
     try {
@@ -535,6 +544,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
         if (k > 0) {
           launch_gcr_multidot(Vh, a, ctx, st);
           const SolverState S = read_state(ctx);
+          require_inner(S);
           for (int j = 0; j < k; j++) {
             // |W_j|^2 was stored when W_j was made
             a.beta[2 * j] = S.sums[2 * j] / nw[j];
@@ -543,7 +553,12 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
           info.iterations += pc == 1 ? 1 : S.iter;  // inner iterations of this step
           if (inner && !nodes) note_launch(2 + per_pass * std::max(S.iter, 1));
         } else {
-          const int it = pc == 1 ? 1 : read_state(ctx).iter;
+          int it = 1;
+          if (pc != 1) {
+            const SolverState S = read_state(ctx);
+            require_inner(S);
+            it = S.iter;
+          }
           info.iterations += it;
           if (inner && !nodes) note_launch(2 + per_pass * std::max(it, 1));
         }
@@ -570,16 +585,6 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
     throw;
   }
   if (inner) cudaGraphExecDestroy(inner);
-  if (small) {  // a wait of the kernel's barriers that gave up
-    int failed = 0;
-    QCU_CUDA(cudaMemcpyAsync(&failed, &ctx.grid_red->failed, sizeof(int), cudaMemcpyDeviceToHost, st));
-    QCU_CUDA(cudaStreamSynchronize(st));
-    if (failed) {
-      QCU_CUDA(cudaMemsetAsync(ctx.grid_red, 0, sizeof(GridRed), st));
-      throw Error(2, "solve: a barrier of the inner solve timed out");
-    }
-  }
-  if (pc == 3) mg_check_coarse(*prm.mg, ctx);
   if (info.status == ST_RUNNING && info.iterations >= prm.maxiter) info.status = ST_MAXITER;
 }
 

@@ -97,38 +97,64 @@ __device__ __forceinline__ Pos step(const Geom &g, Pos c, int d, int st) {
   return c;
 }
 
-// Links staged ahead of their use: every thread copies the rows 0 and 1 of its
-// own links into its own slots of shared memory (cp.async, 16 bytes a lane and
-// row element, so a warp's accesses are contiguous) and reads them back when
-// their turn comes, two links later: no barrier, and no registers held by
-// loads in flight.
+// Links staged ahead of their use: a warp copies the rows 0 and 1 of its 32
+// sites' links into its slots of shared memory (cp.async, 16 bytes a lane) and
+// reads them back when their turn comes, two links later: no block barrier, and
+// no registers held by loads in flight.  Packed links are contiguous over the
+// sites, so every thread copies its own.  Of PyQuda's records (144 bytes apart)
+// a request for one element of 32 sites would touch 32 lines: there the lanes
+// take consecutive pieces of sixteen records at a time, and each reads its own
+// record afterwards (96 bytes apart, rotated by one piece in every second four
+// records against bank conflicts).  dslashCloverQcu needs no packed copy of the
+// links for that: 24^3 x 48 540 us a call, against 629 with a thread per record
+// and 547 when the links were packed first, into 768 B a site more of scratch.
 constexpr int CL_SLOTS = 3;
 constexpr int CL_SLOT_BYTES = 6 * 16 * 32;  // one warp's links
 template <int G>
 struct LinkStage {
   GaugeView<G> U;
   Geom g;
-  unsigned slot0;  // this lane's 16 bytes of element 0 of slot 0
+  unsigned slot0;  // the warp's slot 0
   const double2 *slot0p;
+  int lane;
+  // 16-byte unit of piece p in record r
+  static __device__ __forceinline__ int unit(int r, int p) {
+    p += (r >> 2) & 1;
+    return r * 6 + (p >= 6 ? p - 6 : p);
+  }
+  static __device__ __forceinline__ void copy16(unsigned d, const double2 *p) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(p) : "memory");
+  }
+  // every lane calls it
   __device__ __forceinline__ void fetch(int i, const Pos &c, int mu) const {
     const int s = ((c.t * g.Lz + c.z) * g.Ly + c.y) * g.Lxh + (c.x >> 1);
-    const size_t slab = (size_t)(mu * 2 + ((c.x + c.y + c.z + c.t) & 1)) * U.stride;
-    const double2 *p = static_cast<const double2 *>(U.p) + (G == GAOS64 ? (slab + s) * 9 : slab * 6 + blk_base<6>(s));
+    const int slab = mu * 2 + ((c.x + c.y + c.z + c.t) & 1);
     const unsigned d = slot0 + (i % CL_SLOTS) * CL_SLOT_BYTES;
+    if constexpr (G == GAOS64) {
+      const unsigned l = (unsigned)slab * (unsigned)U.stride + (unsigned)s;  // < 8 * 2^28
+      __syncwarp();  // the link that lay here has been read
 #pragma unroll
-    for (int k = 0; k < 6; k++)
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d + k * 512), "l"(p + (G == GAOS64 ? k : k * SB))
-                   : "memory");
+      for (int k = 0; k < 6; k++) {
+        const int j = (k % 3) * 32 + lane, r = j / 6, p = j % 6;
+        copy16(d + (k / 3) * 16 * 96 + unit(r, p) * 16,
+               static_cast<const double2 *>(U.p) + (size_t)__shfl_sync(0xffffffffu, l, 16 * (k / 3) + r) * 9 + p);
+      }
+    } else {
+      const double2 *p = static_cast<const double2 *>(U.p) + (size_t)slab * U.stride * 6 + blk_base<6>(s);
+#pragma unroll
+      for (int k = 0; k < 6; k++) copy16(d + k * 512 + lane * 16, p + k * SB);
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   // link i, once at most `pending` later fetches are still in flight
   template <int PENDING>
   __device__ __forceinline__ void take(int i, C *m) const {
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+    if constexpr (G == GAOS64) __syncwarp();  // the other lanes' pieces as well
     const double2 *p = slot0p + (i % CL_SLOTS) * (CL_SLOT_BYTES / 16);
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-      const double2 v = p[k * 32];
+      const double2 v = p[G == GAOS64 ? unit(lane, k) : k * 32 + lane];
       m[k] = C(v.x, v.y);
     }
     m[6] = row2(m[1], m[5], m[2], m[4]);
@@ -356,11 +382,11 @@ __global__ void __launch_bounds__(CB_THREADS, 2) k_clover_build(Geom g, GaugeVie
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int s0 = blockIdx.x * groups * SB, q = blockIdx.y;
   const int mu = warp < 3 ? 0 : (warp < 5 ? 1 : 2), nu = warp < 3 ? warp + 1 : (warp < 5 ? warp - 1 : 3);
-  unsigned char *slot = cb_smem + warp * CL_SLOTS * CL_SLOT_BYTES + lane * 16;
-  const LinkStage<G> S{U, g, (unsigned)__cvta_generic_to_shared(slot), reinterpret_cast<const double2 *>(slot)};
+  unsigned char *slot = cb_smem + warp * CL_SLOTS * CL_SLOT_BYTES;
+  const LinkStage<G> S{U, g, (unsigned)__cvta_generic_to_shared(slot), reinterpret_cast<const double2 *>(slot), lane};
   for (int k = 0; k < groups; k++) {
-    const int s = s0 + k * SB + lane;
-    if (s >= g.Vh) break;
+    if (s0 + k * SB >= g.Vh) break;
+    const int s = min(s0 + k * SB + lane, g.Vh - 1);  // lanes past the end copy for the others
     Pos c;
     int xh;
     site_coords(g, s, xh, c.y, c.z, c.t);
@@ -393,7 +419,8 @@ size_t clover_bytes(int ckind, int Vh) { return (size_t)2 * (ckind == CSOA64 ? 1
 void launch_clover_build(int gkind, const Geom &g, const void *gauge, int nparities, double coeff, const CloverOut &o,
                          cudaStream_t s) {
   // three rounds a block once that still fills every SM with its two blocks
-  // (below, the shorter blocks finish sooner than the balance of the last phase gains)
+  // twice (below, the shorter blocks finish sooner than the balance of the last
+  // phase gains)
   const int blocks = (g.Vh + SB - 1) / SB;
   const int groups = (int64_t)blocks * nparities >= 148 * 2 * CB_GROUPS * 2 ? CB_GROUPS : 1;
   const dim3 grid((blocks + groups - 1) / groups, nparities);

@@ -73,7 +73,6 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf();
   void ensure(size_t bytes);  // grow-only
-  bool try_ensure(size_t bytes);  // false (and the buffer empty) where there is no memory for it
   void release();
   template <typename T>
   T *as() const {
@@ -106,11 +105,10 @@ struct Context {
   size_t partials_blocks = 0;
   int sms = 148;                   // multiprocessors of the device
   // scratch of the legacy clover call (dslashCloverQcu): the inverse clover
-  // of the output parity, its zero-pivot counter and the packed links.  Per
-  // device, used only under `mu`; allocated on first use and kept until exit.
+  // of the output parity and its zero-pivot counter.  Per device, used only
+  // under `mu`; allocated on first use and kept until exit.
   DevBuf *legacy_clover = nullptr;
   DevBuf *legacy_bad = nullptr;
-  DevBuf *legacy_gauge = nullptr;
   GridRed *grid_red = nullptr;  // device; the state of cooperative kernels' reductions
   std::mutex mu;
   void ensure_partials(size_t blocks);

@@ -115,22 +115,6 @@ void DevBuf::ensure(size_t bytes) {
   n = bytes;
 }
 
-bool DevBuf::try_ensure(size_t bytes) {
-  if (bytes <= n) return true;
-  release();
-  Context &ctx = context();
-  stream = ctx.stream;
-  const cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool_for(ctx.device), stream);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    p = nullptr;
-    return false;
-  }
-  QCU_CUDA(e);
-  n = bytes;
-  return true;
-}
-
 void Spinor::alloc(int k, int vh) {
   kind = k;
   Vh = vh;

@@ -896,8 +896,6 @@ void handle_mat(GaugeHandle &G, void *out, const void *in, double kappa, int use
 }
 
 // ---------------------------------------------------------------- legacy direct path
-static constexpr int LEGACY_PACK_VH = 32768;  // 16^4, 38 MB of links
-
 void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[4], int parity, int clover) {
   require(out && in && gauge, "dslash: null pointer argument");
   require(parity == 0 || parity == 1, "parity must be 0 or 1");
@@ -912,36 +910,25 @@ void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[
   d.parity = parity;
   d.t_bc = 1.0;
   d.a = 1.0;
-  int gkind = GAOS64;
   if (clover && ctx.legacy_clover == nullptr) {  // this device's scratch, reused across calls, never freed
     ctx.legacy_clover = new DevBuf();
     ctx.legacy_bad = new DevBuf();
-    ctx.legacy_gauge = new DevBuf();
   }
-  DevBuf *cl = ctx.legacy_clover, *bad = ctx.legacy_bad, *packed = ctx.legacy_gauge;
+  DevBuf *cl = ctx.legacy_clover, *bad = ctx.legacy_bad;
   if (clover) {
     // qcu builds the clover of the output parity with unit normalisation on
     // every call (src/nccl_clover_dslash.cu:27-61)
     cl->ensure(clover_bytes(CSOA64, g.Vh));
     bad->ensure(sizeof(int));
     QCU_CUDA(cudaMemsetAsync(bad->p, 0, sizeof(int), ctx.stream));
-    // The build reads every link about 18 times and the hop once more: packing
-    // them first makes those reads contiguous.  It pays where the records do
-    // not stay in L2: 24^3 x 48 569 us a call against 629, 16^4 102 us both.  Without room for the packed copy both read
-    // the caller's records.
-    if (g.Vh > LEGACY_PACK_VH && packed->try_ensure(gauge_bytes(GSOA64, g.Vh))) {
-      launch_gauge_pack(g, gauge, packed->p, nullptr, nullptr, ctx.stream);
-      d.gauge = packed->p;
-      gkind = GSOA64;
-    }
     CloverOut o;
     o.par0 = parity;
     o.Ainv64[0] = cl->p;
     o.bad = bad->as<int>();
-    launch_clover_build(gkind, g, d.gauge, 1, 1.0, o, ctx.stream);
+    launch_clover_build(GAOS64, g, gauge, 1, 1.0, o, ctx.stream);
     d.clover = cl->p;
   }
-  launch_dslash(AOS64, gkind, CSOA64, g, d, ctx, ctx.stream);
+  launch_dslash(AOS64, GAOS64, CSOA64, g, d, ctx, ctx.stream);
   int nbad = 0;
   if (clover) QCU_CUDA(cudaMemcpyAsync(&nbad, bad->p, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
   QCU_CUDA(cudaStreamSynchronize(ctx.stream));

@@ -17,12 +17,21 @@
 //     from the vectors before the update (r and p therefore alternate between
 //     two buffers), while two other warps update the block's own x, r and p;
 //   * <rt, r> = <rt, s> - omega <rt, t> and |r|^2 = |s|^2 - |<t, s>|^2 / |t|^2
-//     of the new residual come with the second product's sums.
+//     of the new residual come with the second product's sums: FP64 sums of FP64
+//     products with t as it is stored, since the differences round relative to
+//     |s|^2 and not to |r|^2.  They hold where one iteration takes |s|^2 down by
+//     less than about 1e15 (beyond, fmax makes |r|^2 zero and the solve ends); the
+//     rounding of t to 16 bits alone leaves |r|^2 at some 1e-11 |s|^2.
 // Vectors are stored in 16 bits and computed in FP32, sums in FP64, as in the
 // kernels of dslash.cu and blas.cu.  A whole solve's time per inner iteration,
-// outer steps included, with clover: 8^3 x 16 58.6 -> 34.7 us, 12^3 x 16 58.7 ->
-// 53.0 us; at 16^4 it would rise from 66 to 91 us, seven tiles a block one after
-// the other, so the graph of kernels keeps more than three tiles an SM.
+// outer steps included, 24 systems each, with the graph of kernels -> with this one:
+//                with the clover term      without
+//   8^3 x 16     57.4 -> 34.4 us           55.0 -> 33.3 us
+//   12^2 x 8 x 16  57.7 -> 43.4            55.5 -> 41.8
+//   12^3 x 16    59.4 -> 53.0              57.0 -> 50.1    (three tiles an SM)
+// at 16^4 it would rise from 66 to 91 us, seven tiles a block one after the other,
+// so the graph of kernels keeps more than three tiles an SM.  (FP32 products in the
+// sums: 33.9 us at 8^3 x 16 with the clover term.)
 #include <algorithm>
 
 #include "gridbar.cuh"
@@ -85,8 +94,10 @@ __device__ __forceinline__ void add_scaled(CF (&v)[N], CF a, const R &r) {
 }
 
 // 16-bit store of one site by two warps (q = chirality): the site's largest
-// component over both goes through mx; bar names a barrier of the two
-__device__ __forceinline__ void store6(void *p, float *n, int s, bool active, int q, const CF (&v)[6], float (*mx)[32],
+// component over both goes through mx; bar names a barrier of the two.  STORED:
+// v becomes what a load of the stored site gives.
+template <bool STORED = false>
+__device__ __forceinline__ void store6(void *p, float *n, int s, bool active, int q, CF (&v)[6], float (*mx)[32],
                                        int bar) {
   const int lane = threadIdx.x & 31;
   float m = 0.f;
@@ -96,14 +107,17 @@ __device__ __forceinline__ void store6(void *p, float *n, int s, bool active, in
   asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
   m = fmaxf(m, mx[1 - q][lane]);
   asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");  // mx may be written again
-  if (!active) return;
   const float k = m > 0.f ? FIX16_SCALE / m : 0.f;
-  unsigned w[6];
+  Raw6 r;
+  r.n = m * F16;
+  unsigned(&w)[6] = r.w;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     w[2 * c] = fix16_pack_k(v[c].re, v[3 + c].re, k);
     w[2 * c + 1] = fix16_pack_k(v[c].im, v[3 + c].im, k);
   }
+  if constexpr (STORED) decode(r, v);
+  if (!active) return;
   char *b = static_cast<char *>(p);
   if (q) {
     *reinterpret_cast<uint2 *>(b + s16_w8(s) + 24) = make_uint2(w[0], w[1]);
@@ -115,15 +129,17 @@ __device__ __forceinline__ void store6(void *p, float *n, int s, bool active, in
   }
 }
 
+// products and sums in FP64: <rt, r> and |r|^2 of a new residual are differences of these
 __device__ __forceinline__ void dot6(const CF (&a)[6], const CF (&b)[6], double &re, double &im) {
-  float sr = 0.f, si = 0.f;
 #pragma unroll
   for (int c = 0; c < 6; c++) {
-    sr += a[c].re * b[c].re + a[c].im * b[c].im;
-    si += a[c].re * b[c].im - a[c].im * b[c].re;
+    re = fma((double)a[c].re, (double)b[c].re, fma((double)a[c].im, (double)b[c].im, re));
+    im = fma((double)a[c].re, (double)b[c].im, fma(-(double)a[c].im, (double)b[c].re, im));
   }
-  re += (double)sr;
-  im += (double)si;
+}
+__device__ __forceinline__ void norm6(const CF (&a)[6], double &n2) {
+#pragma unroll
+  for (int c = 0; c < 6; c++) n2 = fma((double)a[c].re, (double)a[c].re, fma((double)a[c].im, (double)a[c].im, n2));
 }
 
 // This warp's hop (h = 2 mu + (0 forward, 1 backward)): what its projector
@@ -396,16 +412,15 @@ __global__ void __launch_bounds__(IS_THREADS, 1) k_inner_small(InnerArgs a) {
 #pragma unroll
             for (int k = 0; k < 6; k++) w[k] = w[k] * k2 + q[k];
           }
-          store6(dst, dstn, s, active, warp, w, mx[0], 1);
+          store6<true>(dst, dstn, s, active, warp, w, mx[0], 1);
           if (par && active) {
-            double none = 0.0;
             decode(Z, z);
             dot6(z, w, v8[0], v8[1]);  // <rt, v> or <rt, t>
             if (part == 3) {
               dot6(w, q, v8[2], v8[3]);  // <t, s>
-              dot6(w, w, v8[4], none);   // |t|^2
+              norm6(w, v8[4]);           // |t|^2
               dot6(z, q, v8[5], v8[6]);  // <rt, s>
-              dot6(q, q, v8[7], none);   // |s|^2
+              norm6(q, v8[7]);           // |s|^2
             }
           }
         } else if (warp < 4 && fresh) {

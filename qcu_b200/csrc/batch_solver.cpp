@@ -517,7 +517,7 @@ std::vector<SolveInfo> solve_batch(const std::vector<BatchSystem> &sys, const So
         for (int r = 0; r < R; r++) {
           if (!act[r]) continue;
           const double rr = S[r].sums[0];
-          if (!(rr == rr)) info[r].status = ST_NAN, act[r] = 0;
+          if (!(rr <= 1e300)) info[r].status = ST_NAN, act[r] = 0;  // not finite: below the target of an infinite source
           else if (rr <= tol2[r]) info[r].status = ST_CONVERGED, act[r] = 0;
           else if (info[r].iterations >= prm.maxiter) info[r].status = ST_MAXITER, act[r] = 0;
         }

@@ -501,7 +501,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
       d64(0, w.x64, w.tmp64, clov, 1.0);
       d64(1, w.tmp64, w.r64, clov, k2, &w.bp, 1.0, &w.x64, -1.0, RED_NORM, FIN_STORE);
       double rr = read_state(ctx).sums[0];
-      if (!(rr == rr)) {
+      if (!(rr <= 1e300)) {  // not finite (an infinite rr would neither converge nor stall)
         info.status = ST_NAN;
         break;
       }

@@ -55,3 +55,20 @@ def test_inner_solve_without_a_result(q, clover, scale):
         b[0].flat[7] = 0  # and nothing of it stays
         info = G.invert(x, dev(b), kappa, **kw)
         assert info["status"] == 1 and info["fallback"] == 0, info
+
+
+@pytest.mark.parametrize("solver,precision", [("gcr", 16), ("gcr", 32), ("bicgstab", 16), ("bicgstab", 64), ("batch", 16)])
+@pytest.mark.parametrize("half", [0, 1])
+def test_source_with_an_infinity_ends(q, solver, precision, half):
+    """|b|^2 and the target are infinite, so no residual is above the target and no cycle counts as stalled."""
+    latt, kappa = [4, 4, 4, 4], 0.12
+    U = O.gauge_smooth(latt, 0.3, 83)
+    b = O.fermion_gauss(O.full_shape(latt), 84)
+    b[half].flat[7] = np.inf
+    x = empty_like_dev(O.full_shape(latt))
+    with q.Gauge(dev(U), latt, t_boundary=-1.0) as G:
+        if solver == "batch":
+            info = q.invert_batch([(G, x[None], dev(b[None]), kappa, False)], tol=1e-10, maxiter=400, precision=16)[0][0]
+        else:
+            info = G.invert(x, dev(b), kappa, tol=1e-10, maxiter=400, solver=solver, precision=precision)
+    assert info["status"] == 4, info

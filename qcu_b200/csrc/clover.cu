@@ -417,12 +417,12 @@ __global__ void k_clover_apply(int Vh, CloverView<CSOA64> cv, const void *in, vo
 size_t clover_bytes(int ckind, int Vh) { return (size_t)2 * (ckind == CSOA64 ? 18 * 16 : 9 * 16) * pad_sites(Vh); }
 
 void launch_clover_build(int gkind, const Geom &g, const void *gauge, int nparities, double coeff, const CloverOut &o,
-                         cudaStream_t s) {
+                         int sms, cudaStream_t s) {
   // three rounds a block once that still fills every SM with its two blocks
   // twice (below, the shorter blocks finish sooner than the balance of the last
   // phase gains)
   const int blocks = (g.Vh + SB - 1) / SB;
-  const int groups = (int64_t)blocks * nparities >= 148 * 2 * CB_GROUPS * 2 ? CB_GROUPS : 1;
+  const int groups = (int64_t)blocks * nparities >= (int64_t)sms * 2 * CB_GROUPS * 2 ? CB_GROUPS : 1;
   const dim3 grid((blocks + groups - 1) / groups, nparities);
   auto run = [&](auto kernel, auto view) {
     QCU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CB_SMEM));

@@ -24,7 +24,7 @@
 
 namespace qcu {
 
-constexpr int GRID_RED_BLOCKS = 148 * 4;  // at most
+constexpr int GRID_RED_BLOCKS = 592;  // room for so many blocks (four an SM); a launch takes no more
 constexpr int GRID_RED_VALUES = 8;    // sums of one reduction, at most
 struct GridRed {
   unsigned count;  // arrivals

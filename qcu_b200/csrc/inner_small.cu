@@ -532,7 +532,8 @@ __global__ void __launch_bounds__(IS_THREADS, 1) k_inner_small(InnerArgs a) {
 
 }  // namespace
 
-bool inner_small_fits(int Vh) { return Vh <= INNER_SMALL_VH; }
+// three 32-site tiles an SM: beyond, the graph of kernels overtakes it
+bool inner_small_fits(int Vh, int sms) { return Vh <= 3 * 32 * sms; }
 
 void launch_inner_small(const InnerArgs &a, int sms, cudaStream_t s) {
   const int grid = std::min(std::min(GRID_RED_BLOCKS, sms), (a.g.Vh + 31) / 32);  // one block an SM

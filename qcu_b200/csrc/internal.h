@@ -204,8 +204,7 @@ struct InnerArgs {
   SolverState *st = nullptr;
   GridRed *red = nullptr;
 };
-constexpr int INNER_SMALL_VH = 3 * 148 * 32;  // three 32-site tiles an SM: where the graph of kernels overtakes it
-bool inner_small_fits(int Vh);
+bool inner_small_fits(int Vh, int sms);
 void launch_inner_small(const InnerArgs &a, int sms, cudaStream_t s);
 void launch_convert(int kin, int kout, int Vh, const void *in, const float *in_n, void *out, float *out_n,
                     cudaStream_t s);
@@ -228,7 +227,7 @@ struct CloverOut {
   int *bad = nullptr;  // counts blocks with a zero pivot
 };
 void launch_clover_build(int gkind, const Geom &g, const void *gauge, int nparities, double coeff, const CloverOut &o,
-                         cudaStream_t s);
+                         int sms, cudaStream_t s);
 // out = C in for a packed clover C (AOS64 or SOA64 spinors)
 void launch_clover_apply(int kind, int Vh, const void *c64, const void *in, void *out, cudaStream_t s);
 size_t clover_bytes(int ckind, int Vh);

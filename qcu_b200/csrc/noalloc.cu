@@ -73,7 +73,8 @@ void clover_dslash_noalloc(void *out, const void *in, const void *gauge, const i
   o.par0 = parity;
   o.Ainv64[0] = slot.clover;
   o.bad = slot.bad;
-  launch_clover_build(GAOS64, g, gauge, 1, 1.0, o, s);
+  Context none;  // no reductions: the launches touch neither solver state nor partials
+  launch_clover_build(GAOS64, g, gauge, 1, 1.0, o, none.sms, s);
   DslashArgs d;
   d.in = in;
   d.out = out;
@@ -82,7 +83,6 @@ void clover_dslash_noalloc(void *out, const void *in, const void *gauge, const i
   d.t_bc = 1.0;
   d.a = 1.0;
   d.clover = slot.clover;
-  Context none;  // no reductions: the launch touches neither solver state nor partials
   launch_dslash(AOS64, GAOS64, CSOA64, g, d, none, s);
   int nbad = 0;
   QCU_CUDA(cudaMemcpyAsync(&nbad, slot.bad, sizeof(int), cudaMemcpyDeviceToHost, s));

@@ -65,7 +65,7 @@ GaugeHandle *gauge_load(const void *gauge_pyq, const int latt[4], double t_bc, d
         o.Ainv64[p] = G->Ainv64[p].p;
         o.Ainv32[p] = G->Ainv32[p].p;
       }
-      launch_clover_build(GSOA64, G->g, G->g64.p, 2, clover_coeff, o, ctx.stream);
+      launch_clover_build(GSOA64, G->g, G->g64.p, 2, clover_coeff, o, ctx.sms, ctx.stream);
       int nbad = 0;
       QCU_CUDA(cudaMemcpyAsync(&nbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
       QCU_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -445,7 +445,7 @@ static void run_gcr(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &vs, const Sol
   long long per_pass = 0;  // kernels per pass of the WHILE body
   cudaGraphExec_t inner = nullptr;
   // 16-bit inner solves of small lattices: one cooperative kernel instead of a graph
-  const bool small = pc != 1 && dP.kind == SOA16 && inner_small_fits(Vh);
+  const bool small = pc != 1 && dP.kind == SOA16 && inner_small_fits(Vh, ctx.sms);
   InnerArgs ia;
   if (small) {
     ia.g = dP.G.g;
@@ -925,7 +925,7 @@ void legacy_dslash(void *out, const void *in, const void *gauge, const int latt[
     o.par0 = parity;
     o.Ainv64[0] = cl->p;
     o.bad = bad->as<int>();
-    launch_clover_build(GAOS64, g, gauge, 1, 1.0, o, ctx.stream);
+    launch_clover_build(GAOS64, g, gauge, 1, 1.0, o, ctx.sms, ctx.stream);
     d.clover = cl->p;
   }
   launch_dslash(AOS64, GAOS64, CSOA64, g, d, ctx, ctx.stream);

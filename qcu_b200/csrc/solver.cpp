@@ -293,10 +293,17 @@ static cudaGraphNode_t add_step_loop(cudaGraph_t g, const cudaGraphNode_t *after
   QCU_CUDA(cudaStreamEndCapture(st, &body));
   return loop;
 }
-// The BiCGSTAB loop, up to its end or the next reliable update, as a graph.  (A
-// graph of 8 to 32 unrolled iterations takes as long to instantiate as several
-// of them to run on a small lattice, and launches four gated kernels an
-// iteration for an update that comes once in dozens.)
+// The BiCGSTAB loop, up to its end or the next reliable update, as a graph, up to
+// a limit on delta.  A graph of 8 to 32 unrolled iterations takes as long to
+// instantiate as several of them to run on a small lattice, and launches four
+// gated kernels an iteration for an update that comes once in dozens; but this
+// one returns to the host for every update, and where the residual is taken
+// afresh whenever it has dropped by a little, the gated kernels cost less.  Time
+// against the unrolled graphs (64, 32 and 16 bits, two kappa):
+//   delta            0.1        0.3        0.5        0.7        0.9
+//   4^4 - 12^3 x 16  0.73-0.92  0.77-0.96  0.84-0.99  0.90-1.05  0.94-1.11
+//   16^4 - 24^3 x 48 0.88-0.99  0.91-1.00  0.98-1.02  0.99-1.07  1.00-1.15
+static double while_delta(int Vh) { return Vh >= (1 << 14) ? 0.4 : 0.6; }
 static cudaGraphExec_t capture_bicgstab(Dsl &dP, Workspace &w, const VecSet &vs, double kappa, bool clov,
                                         long long &per_pass) {
   cudaStream_t st = dP.ctx.stream;
@@ -613,12 +620,12 @@ static SolverState run_bicgstab(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &v
   if (!S.done) {
     cudaGraphExec_t exec = nullptr;
     long long nodes = 0;
-    if (use_graph && prm.chunk == 0) {
+    if (use_graph && prm.chunk == 0 && prm.delta <= while_delta(Vh)) {
       long long per_pass = 0;
       try {
         exec = capture_bicgstab(dP, w, vs, kappa, clov, per_pass);
       } catch (const Error &) {
-        exec = nullptr;  // conditional graph nodes unavailable: unrolled graphs of `chunk` iterations
+        exec = nullptr;  // conditional graph nodes unavailable: unrolled graphs
       }
       if (exec) {
         try {
@@ -638,7 +645,7 @@ static SolverState run_bicgstab(Dsl &dP, Dsl &d64, Workspace &w, const VecSet &v
         exec = nullptr;
       }
     }
-    if (!S.done && use_graph) {
+    if (!S.done && use_graph) {  // unrolled: `chunk` iterations and their gated updates
       cudaGraph_t graph;
       const long long before = launch_count();
       QCU_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));

@@ -468,7 +468,7 @@ struct CoarseArgs {
   CState *st;
   double tol2;
   int maxit;
-  int apb;  // aggregates a block works on at a time: 1, 2 or 4
+  int apb;  // aggregates a block works on at a time, a power of two
 };
 
 // x ~ A_c^-1 b by BiCGSTAB (FP32 vectors, FP64 scalars) from zero, to
@@ -480,29 +480,48 @@ struct CoarseArgs {
 // |r|^2 of the new residual r = s - omega t follow from the products of s, t
 // and rt that the second application's reduction carries,
 //   <rt, r> = <rt, s> - omega <rt, t>,   |r|^2 = |s|^2 - |<t, s>|^2 / |t|^2.
-// The 32 warps of a block share the columns of 1, 2 or 4 aggregates (lane =
+// The 32 warps of a block share the columns of one or more aggregates (lane =
 // row).  Bound by the latency of its barriers and of A_c's entries from L2
 // (where every block's part fits, it stays in shared memory).  16^3 x 32, 4^4
 // aggregates, 24 rows: 12.8 us an iteration, 4.3 of them the barriers, where
 // nine kernels an iteration took 49 us.
 // A_c larger than MGC_STREAM is read from HBM, and the chain from an aggregate's
 // neighbours to its inputs to its product has to be covered: four blocks of 256
-// threads an SM, each with an aggregate of its own at its own place in the chain,
-// and the next aggregate's matrix asked for ahead.  32^3 x 64 (340 MB): 165 us an
+// threads an SM, each at its own place in the chain, and the next aggregate's
+// matrix asked for ahead.  32^3 x 64 (340 MB): 165 us an
 // iteration, against 226 with one block of 1024 (211 with four blocks but nothing
 // asked for ahead) and 181 with nine kernels; 24^3 x 48 (108 MB): 70, 89 and 91.
+// Aggregates with few rows are many and their matrices small: a block takes as
+// many at a time as have the threads for their inputs (mgc_threads), and where a
+// warp or two are left to each, the lanes share a row's columns as well (SPLIT).
+// us an iteration, aggregates x rows: nine kernels / four (one when streamed) a
+// block, lane = row / as now:
+//   4096 x 4 (5 MB)     35 /  41 / 15        20736 x 8 (96 MB)    122 / 215 /  89
+//   4096 x 8 (19 MB)    39 /  44 / 26        65536 x 4 (75 MB)    190 / 512 / 124
+//   8192 x 8 (38 MB)    56 /  80 / 42         8192 x 16 (151 MB)  130 / 133 /  97
+// (With a whole block an aggregate the shares are too many to sum: 128 x 8 11.0 ->
+// 21.4 us, so SPLIT only comes with the fewest threads; with 24 rows one lane a
+// row and 256 threads an aggregate are faster: 1296 x 24 34.7 us, 42.9 split and
+// 37.5 with 128; 2592 x 24, streamed, 69, 76 and 74.)
 constexpr int MGC_THREADS = 1024;
 // below it the one large block is as fast (24^4, 54 MB: 35 us against 37; 16^2 x
 // 24 x 32: 27 against 30), as the matrices stay in L2
 constexpr size_t MGC_STREAM = (size_t)64 << 20;
 constexpr int MGC_SMEM = 180 * 1024;  // the most a block's matrices may take of its shared memory
-template <bool CACHED, int T>
+// the fewest threads an aggregate of nc rows takes: two of its 9 nc inputs each
+int mgc_threads(int nc) {
+  if (nc > 16) return 256;
+  int t = 32;
+  while (2 * t < 9 * nc) t *= 2;
+  return t;
+}
+template <bool CACHED, int T, bool SPLIT>
 __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) {
   constexpr bool STREAM = T < MGC_THREADS;
   extern __shared__ float4 ysm[];  // CACHED: the entries of the block's aggregates
-  __shared__ float2 xin[T / 256][9 * 2 * MG_MAXVEC];
+  __shared__ float2 xin_all[2 * T];  // [aggregate][J]: at most two inputs a thread
   __shared__ float2 psum[T / 32][32];
-  __shared__ int nb[T / 256][9];
+  __shared__ int nb[T / 32][9];
   __shared__ GridRedShared red;
   __shared__ double tot[8];
   __shared__ double2 sc[5];  // alpha, omega, beta, beta omega, rho
@@ -510,10 +529,14 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
   const int nc = a.m.nc, J = 9 * nc, P = J / 2;
   const int tpa = T / a.apb, wpa = tpa / 32;
   const int al = threadIdx.x / tpa, lt = threadIdx.x % tpa, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float2 *const xin = xin_all + al * J;
   const int first = blockIdx.x * a.apb, stride = gridDim.x * a.apb;
   if (grid_red_failed(&a.st->red)) return;
-  const int jp0 = (lt >> 5) * P / wpa, jp1 = ((lt >> 5) + 1) * P / wpa;
-  // the (at most two, as J <= 288 and tpa >= 256) inputs this thread stages: block d, row
+  // SPLIT: lane = row + nc * (its share of the warp's columns); else lane = row
+  const int groups = SPLIT ? 32 / nc : 1, grp = SPLIT ? lane / nc : 0, row = SPLIT ? lane - grp * nc : lane;
+  const int parts = wpa * groups, share = (lt >> 5) * groups + grp;
+  const int jp0 = share * P / parts, jp1 = (share + 1) * P / parts;
+  // the (at most two, as J <= 2 tpa) inputs this thread stages: block d, row
   const int d0 = lt / nc, row0 = lt - d0 * nc, d1 = (lt + tpa) / nc, row1 = lt + tpa - d1 * nc;
   const unsigned count0 = a.st->red.base;
   unsigned epoch = 0;
@@ -521,14 +544,21 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
   // A_c times the staged inputs at row lt < nc of aggregate B (every thread calls it)
   auto apply = [&](int B, bool mine) -> float2 {
     __syncthreads();
-    if (mine && lane < nc)
-      psum[warp][lane] = CACHED ? mg_row<true>(ysm + (size_t)al * P * nc + lane, nc, xin[al], jp0, jp1)
-                       : STREAM ? mg_row_wide<7>(a.Y + (size_t)B * P * nc + lane, nc, xin[al], jp0, jp1)
-                                : mg_row<false>(a.Y + (size_t)B * P * nc + lane, nc, xin[al], jp0, jp1);
+    if (mine && (SPLIT ? grp < groups : lane < nc))
+      psum[warp][lane] = CACHED ? mg_row<true>(ysm + (size_t)al * P * nc + row, nc, xin, jp0, jp1)
+                       : STREAM ? mg_row_wide<7>(a.Y + (size_t)B * P * nc + row, nc, xin, jp0, jp1)
+                                : mg_row<false>(a.Y + (size_t)B * P * nc + row, nc, xin, jp0, jp1);
     __syncthreads();
     float2 o = make_float2(0.f, 0.f);
     if (mine && lt < nc)
-      for (int w = 0; w < wpa; w++) o = make_float2(o.x + psum[al * wpa + w][lt].x, o.y + psum[al * wpa + w][lt].y);
+      for (int w = 0; w < wpa; w++) {
+        if constexpr (SPLIT) {
+          for (int k = lt; k < groups * nc; k += nc)
+            o = make_float2(o.x + psum[al * wpa + w][k].x, o.y + psum[al * wpa + w][k].y);
+        } else {
+          o = make_float2(o.x + psum[al * wpa + w][lt].x, o.y + psum[al * wpa + w][lt].y);
+        }
+      }
     return o;
   };
   auto neighbours = [&](int B) {
@@ -538,7 +568,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
   // after the last) fetched into L2 while B's inputs are formed and used
   auto prefetch = [&](int B) {
     const int Bn = B + stride < a.m.nblocks ? B + stride : first + al;
-    if (STREAM && lt == 32 && Bn < a.m.nblocks)
+    if (STREAM && lt == tpa - 1 && Bn < a.m.nblocks)
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.Y + (size_t)Bn * P * nc), "r"(P * nc * 16) : "memory");
   };
 
@@ -599,7 +629,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
                                  x.y + ar * p.y + ai * p.x + wr * s.y + wi * s.x);
           }
         }
-        xin[al][i] = pn;
+        xin[i] = pn;
         if (d == 8) {
           rc[e] = rn;
           pc[e] = pn;
@@ -641,7 +671,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
       auto stage = [&](int i, int d, int row) {
         const size_t e = (size_t)nb[al][d] * nc + row;
         const float2 r = __ldcg(rc + e), q = __ldcg(vc + e);
-        xin[al][i] = make_float2(r.x - ar * q.x + ai * q.y, r.y - ar * q.y - ai * q.x);
+        xin[i] = make_float2(r.x - ar * q.x + ai * q.y, r.y - ar * q.y - ai * q.x);
       };
       if (mine && lt < J) stage(lt, d0, row0);
       if (mine && lt + tpa < J) stage(lt + tpa, d1, row1);
@@ -649,7 +679,7 @@ __global__ void __launch_bounds__(T, MGC_THREADS / T) k_mg_coarse(CoarseArgs a) 
       if (mine && lt < nc) {
         const size_t e = (size_t)B * nc + lt;
         a.t[e] = o;
-        const float2 s = xin[al][8 * nc + lt], q = a.b[e];
+        const float2 s = xin[8 * nc + lt], q = a.b[e];
         v8[0] += (double)o.x * s.x + (double)o.y * s.y;  // <t, s>
         v8[1] += (double)o.x * s.y - (double)o.y * s.x;
         v8[2] += (double)o.x * o.x + (double)o.y * o.y;  // |t|^2
@@ -1008,16 +1038,21 @@ void coarse_solve(MG &mg, Context &ctx) {
   a.maxit = mg.p.coarse_maxiter;
   const size_t part = (size_t)(9 * a.m.nc / 2) * a.m.nc * sizeof(float4);  // of A_c, an aggregate's
   const bool stream = part * mg.m.nblocks > MGC_STREAM;
-  const int T = stream ? 256 : MGC_THREADS, per = MGC_THREADS / T;
+  const int T = stream ? 256 : MGC_THREADS, per = MGC_THREADS / T, fewest = mgc_threads(a.m.nc);
   // spread the aggregates over the SMs before a block takes several at a time
-  a.apb = stream || mg.m.nblocks <= ctx.sms ? 1 : (mg.m.nblocks <= 2 * ctx.sms ? 2 : 4);
+  a.apb = stream ? T / fewest : 1;
+  while (!stream && a.apb * ctx.sms < mg.m.nblocks && T / (2 * a.apb) >= fewest) a.apb *= 2;
+  const bool split = T / a.apb == fewest && a.m.nc <= 16;
   const int grid = std::min(std::min(per * ctx.sms, GRID_RED_BLOCKS), (mg.m.nblocks + a.apb - 1) / a.apb);
   // A_c stays in shared memory where every block has one set of aggregates that fits
   const size_t smem = a.apb * part;
   const bool cached = !stream && smem <= MGC_SMEM && (int64_t)grid * a.apb >= a.m.nblocks;
-  const void *k = stream   ? reinterpret_cast<const void *>(k_mg_coarse<false, 256>)
-                  : cached ? reinterpret_cast<const void *>(k_mg_coarse<true, MGC_THREADS>)
-                           : reinterpret_cast<const void *>(k_mg_coarse<false, MGC_THREADS>);
+  auto pick = [&](auto plain, auto shared_out) {
+    return split ? reinterpret_cast<const void *>(shared_out) : reinterpret_cast<const void *>(plain);
+  };
+  const void *k = stream   ? pick(k_mg_coarse<false, 256, false>, k_mg_coarse<false, 256, true>)
+                  : cached ? pick(k_mg_coarse<true, MGC_THREADS, false>, k_mg_coarse<true, MGC_THREADS, true>)
+                           : pick(k_mg_coarse<false, MGC_THREADS, false>, k_mg_coarse<false, MGC_THREADS, true>);
   if (cached) QCU_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MGC_SMEM));
   void *args[] = {&a};
   QCU_CUDA(grid_red_inject(&a.st->red, "coarse", ctx.stream));

@@ -15,8 +15,8 @@ size_t mrhs_bytes(int Vh, int nrhs);
 void launch_mrhs_tc(const Geom &g, const void *gauge16, double t_bc, const void *in, void *out, int nrhs, int par,
                     int *err, int sms, cudaStream_t s);
 // PyQuda half spinors [nrhs][Vh][12] complex128 <-> multi-rhs FP16 field
-void launch_mrhs_pack(const void *pyq, void *mrhs, int Vh, int nrhs, cudaStream_t s);
-void launch_mrhs_unpack(const void *mrhs, void *pyq, int Vh, int nrhs, cudaStream_t s);
+void launch_mrhs_pack(const void *pyq, void *mrhs, int Vh, int nrhs, int sms, cudaStream_t s);
+void launch_mrhs_unpack(const void *mrhs, void *pyq, int Vh, int nrhs, int sms, cudaStream_t s);
 void launch_mrhs_random(void *mrhs, int Vh, int nrhs, unsigned long long seed, cudaStream_t s);
 
 // on a gauge handle: the operator on PyQuda-layout fields, and the kernel's

@@ -475,7 +475,10 @@ __global__ void __launch_bounds__(MT_THREADS, MtShape<RP>::CTAS_PER_SM) k_mrhs_t
 // nor the 16-byte ones down the rows conflict.  (One thread per 16-byte chunk
 // instead reads and writes the PyQuda side in 64-byte pieces: 16^3 x 32, 64
 // right-hand sides, 1.01 GB each: pack 488 -> 154 us, unpack 990 -> 160 us,
-// 6.3-6.5 TB/s.)
+// 6.3-6.5 TB/s.)  On lattices with fewer tiles than multiprocessors a block
+// takes NR = 16 of the rows (blockIdx.y), two a warp, as its time is then that
+// of the rows one after the other: a call at 4^4 with 128 right-hand sides 46.7 ->
+// 42.2 us (45.0 with a thread per chunk), 8^2 x 4^2 54.6 -> 45.9.
 constexpr int MP_THREADS = 256;
 template <int RP>
 struct MpShape {
@@ -484,14 +487,16 @@ struct MpShape {
 };
 
 // rows beyond nrhs are written as zeros
-template <int RP>
+template <int RP, int NR>
 __global__ void __launch_bounds__(MP_THREADS) k_mrhs_pack(const double2 *in, __half *out, int Vh, int nrhs) {
   constexpr int MP_SITES = MpShape<RP>::SITES, MP_PITCH = MpShape<RP>::PITCH;
-  __shared__ __align__(16) unsigned char sm[RP * MP_PITCH];
-  const int s0 = blockIdx.x * MP_SITES, ns = min(MP_SITES, Vh - s0);
+  __shared__ __align__(16) unsigned char sm[NR * MP_PITCH];
+  const int s0 = blockIdx.x * MP_SITES, ns = min(MP_SITES, Vh - s0), r0 = NR == RP ? 0 : blockIdx.y * NR;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  in += (size_t)r0 * Vh * 12;
+  nrhs -= r0;
 #pragma unroll 2
-  for (int r = warp; r < RP; r += MP_THREADS / 32) {
+  for (int r = warp; r < NR; r += MP_THREADS / 32) {
     uint32_t *row = reinterpret_cast<uint32_t *>(sm + r * MP_PITCH);
     const double2 *p = in + ((size_t)r * Vh + s0) * 12;
 #pragma unroll
@@ -505,21 +510,23 @@ __global__ void __launch_bounds__(MP_THREADS) k_mrhs_pack(const double2 *in, __h
     }
   }
   __syncthreads();
-  uint4 *o = reinterpret_cast<uint4 *>(out) + (size_t)s0 * 3 * RP;
-  for (int i = threadIdx.x; i < ns * 3 * RP; i += MP_THREADS)
-    o[i] = *reinterpret_cast<const uint4 *>(sm + (i % RP) * MP_PITCH + (i / RP) * 16);
+  uint4 *o = reinterpret_cast<uint4 *>(out) + (size_t)s0 * 3 * RP + r0;
+  for (int i = threadIdx.x; i < ns * 3 * NR; i += MP_THREADS)
+    o[NR == RP ? i : i / NR * RP + i % NR] = *reinterpret_cast<const uint4 *>(sm + (i % NR) * MP_PITCH + (i / NR) * 16);
 }
 
-template <int RP>
+template <int RP, int NR>
 __global__ void __launch_bounds__(MP_THREADS) k_mrhs_unpack(const __half *in, double2 *out, int Vh, int nrhs) {
   constexpr int MP_SITES = MpShape<RP>::SITES, MP_PITCH = MpShape<RP>::PITCH;
-  __shared__ __align__(16) unsigned char sm[RP * MP_PITCH];
-  const int s0 = blockIdx.x * MP_SITES, ns = min(MP_SITES, Vh - s0);
+  __shared__ __align__(16) unsigned char sm[NR * MP_PITCH];
+  const int s0 = blockIdx.x * MP_SITES, ns = min(MP_SITES, Vh - s0), r0 = NR == RP ? 0 : blockIdx.y * NR;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint4 *f = reinterpret_cast<const uint4 *>(in) + (size_t)s0 * 3 * RP;
+  const uint4 *f = reinterpret_cast<const uint4 *>(in) + (size_t)s0 * 3 * RP + r0;
+  out += (size_t)r0 * Vh * 12;
+  if (NR != RP) nrhs = min(nrhs - r0, NR);
 #pragma unroll 4
-  for (int i = threadIdx.x; i < ns * 3 * RP; i += MP_THREADS)
-    if (i % RP < nrhs) *reinterpret_cast<uint4 *>(sm + (i % RP) * MP_PITCH + (i / RP) * 16) = __ldcs(f + i);
+  for (int i = threadIdx.x; i < ns * 3 * NR; i += MP_THREADS)
+    if (i % NR < nrhs) *reinterpret_cast<uint4 *>(sm + (i % NR) * MP_PITCH + (i / NR) * 16) = __ldcs(f + (NR == RP ? i : i / NR * RP + i % NR));
   __syncthreads();
   for (int r = warp; r < nrhs; r += MP_THREADS / 32) {
     const uint32_t *row = reinterpret_cast<const uint32_t *>(sm + r * MP_PITCH);
@@ -597,23 +604,35 @@ void launch_mrhs_tc(const Geom &g, const void *gauge16, double t_bc, const void 
   else launch_mt<128>(a, sms, s);
 }
 
-static unsigned mp_blocks(int Vh, int nrhs) {
-  const int sites = mrhs_rows(nrhs) == 64 ? MpShape<64>::SITES : MpShape<128>::SITES;
-  return (unsigned)((Vh + sites - 1) / sites);
+// one block per tile of sites, or, with fewer tiles than multiprocessors, per 16 rows of one
+template <int RP, typename F, typename G>
+static void mp_launch(int Vh, int sms, F whole, G part) {
+  const unsigned tiles = (unsigned)((Vh + MpShape<RP>::SITES - 1) / MpShape<RP>::SITES);
+  if (tiles >= (unsigned)sms) whole(dim3(tiles));
+  else part(dim3(tiles, RP / 16));
+  QCU_CHECK_LAUNCH();
 }
-void launch_mrhs_pack(const void *pyq, void *mrhs, int Vh, int nrhs, cudaStream_t s) {
+template <int RP>
+static void mp_pack(const double2 *in, __half *out, int Vh, int nrhs, int sms, cudaStream_t s) {
+  mp_launch<RP>(Vh, sms, [&](dim3 g) { k_mrhs_pack<RP, RP><<<g, MP_THREADS, 0, s>>>(in, out, Vh, nrhs); },
+                [&](dim3 g) { k_mrhs_pack<RP, 16><<<g, MP_THREADS, 0, s>>>(in, out, Vh, nrhs); });
+}
+template <int RP>
+static void mp_unpack(const __half *in, double2 *out, int Vh, int nrhs, int sms, cudaStream_t s) {
+  mp_launch<RP>(Vh, sms, [&](dim3 g) { k_mrhs_unpack<RP, RP><<<g, MP_THREADS, 0, s>>>(in, out, Vh, nrhs); },
+                [&](dim3 g) { k_mrhs_unpack<RP, 16><<<g, MP_THREADS, 0, s>>>(in, out, Vh, nrhs); });
+}
+void launch_mrhs_pack(const void *pyq, void *mrhs, int Vh, int nrhs, int sms, cudaStream_t s) {
   const double2 *in = static_cast<const double2 *>(pyq);
-  const unsigned blocks = mp_blocks(Vh, nrhs);
-  if (mrhs_rows(nrhs) == 64) k_mrhs_pack<64><<<blocks, MP_THREADS, 0, s>>>(in, static_cast<__half *>(mrhs), Vh, nrhs);
-  else k_mrhs_pack<128><<<blocks, MP_THREADS, 0, s>>>(in, static_cast<__half *>(mrhs), Vh, nrhs);
-  QCU_CHECK_LAUNCH();
+  __half *out = static_cast<__half *>(mrhs);
+  if (mrhs_rows(nrhs) == 64) mp_pack<64>(in, out, Vh, nrhs, sms, s);
+  else mp_pack<128>(in, out, Vh, nrhs, sms, s);
 }
-void launch_mrhs_unpack(const void *mrhs, void *pyq, int Vh, int nrhs, cudaStream_t s) {
+void launch_mrhs_unpack(const void *mrhs, void *pyq, int Vh, int nrhs, int sms, cudaStream_t s) {
   const __half *in = static_cast<const __half *>(mrhs);
-  const unsigned blocks = mp_blocks(Vh, nrhs);
-  if (mrhs_rows(nrhs) == 64) k_mrhs_unpack<64><<<blocks, MP_THREADS, 0, s>>>(in, static_cast<double2 *>(pyq), Vh, nrhs);
-  else k_mrhs_unpack<128><<<blocks, MP_THREADS, 0, s>>>(in, static_cast<double2 *>(pyq), Vh, nrhs);
-  QCU_CHECK_LAUNCH();
+  double2 *out = static_cast<double2 *>(pyq);
+  if (mrhs_rows(nrhs) == 64) mp_unpack<64>(in, out, Vh, nrhs, sms, s);
+  else mp_unpack<128>(in, out, Vh, nrhs, sms, s);
 }
 void launch_mrhs_random(void *mrhs, int Vh, int nrhs, unsigned long long seed, cudaStream_t s) {
   const int RP = mrhs_rows(nrhs);
@@ -649,9 +668,9 @@ void handle_dslash_mrhs(GaugeHandle &G, void *out, const void *in, int nrhs, int
   w.err.ensure(sizeof(int));
   QCU_CUDA(cudaDeviceSynchronize());
   QCU_CUDA(cudaMemsetAsync(w.err.p, 0, sizeof(int), ctx.stream));
-  launch_mrhs_pack(in, w.in.p, Vh, nrhs, ctx.stream);
+  launch_mrhs_pack(in, w.in.p, Vh, nrhs, ctx.sms, ctx.stream);
   launch_mrhs_tc(G.g, G.g16.p, G.t_bc, w.in.p, w.out.p, nrhs, par, w.err.as<int>(), ctx.sms, ctx.stream);
-  launch_mrhs_unpack(w.out.p, out, Vh, nrhs, ctx.stream);
+  launch_mrhs_unpack(w.out.p, out, Vh, nrhs, ctx.sms, ctx.stream);
   mrhs_check_err(w, ctx.stream);
 }
 

@@ -18,11 +18,13 @@
 //   k_tr_odd    out = sum_h T_h z_h + W2[0] W1[0] r, the loss, delta, S
 //   k_tr_outer  R, as a GEMM over (site, colour) in shared memory
 //   k_tr_reduce, k_tr_grads
-// FP32 arithmetic on paired instructions, every sum across blocks in FP64 and
-// in a fixed order (the gradient is reproducible to the bit).  16^4, batch 16:
-// 1.00 ms a step (load 45 us, even 335, odd 144, outer 409), where layer by
-// layer gradients with warp reductions and atomics took 8.2 ms; error of the
-// gradient against 64 bits 3e-8, was 9e-7.
+// FP32 arithmetic on paired instructions; a block's sums of R, S and the loss
+// over its tiles are FP32, the sums across blocks FP64, all in a fixed order (the
+// gradient is reproducible to the bit).  16^4, batch 16: 1.00 ms a step (load 45
+// us, even 335, odd 144, outer 409), where layer by layer gradients with warp
+// reductions and atomics took 8.2 ms.  Error of the gradient against 64 bits, 16^4
+// batch 16, 16^3 x 32 batch 32 and 32^3 x 64 batch 4 (55, 221 and 443 tiles a
+// block): 3.1e-8, 2.9e-8 and 2.8e-8, where it was 9e-7, 1.9e-6 and 2.7e-6.
 #include <algorithm>
 
 #include "hop32.cuh"

@@ -12,7 +12,6 @@ using F2 = float2;
 __device__ __forceinline__ F2 cmul(F2 a, F2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ __forceinline__ F2 cadd(F2 a, F2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 
-
 // neighbour of site s (parity par) in direction mu, step +-1; also whether
 // the hop crosses the t boundary
 __device__ __forceinline__ int nbr(const Geom &g, int s, int par, int mu, int fwd, bool &tcross) {
@@ -41,13 +40,12 @@ __device__ __forceinline__ int nbr(const Geom &g, int s, int par, int mu, int fw
 // read from `in` on the neighbouring site.  Returns false if the hop's source
 // parity holds no input (in_mask).
 template <int CIN>
-__device__ __forceinline__ bool transport(const Geom &g, const PtcArgs &a, const float2 *in_sample, int s, int par,
-                                          int h, F2 v[CIN][3]) {
+__device__ __forceinline__ bool transport(const Geom &g, const PtcArgs &a, int s, int par, int h, F2 v[CIN][3]) {
   const int src_par = h == 0 ? par : 1 - par;
   if (!(a.in_mask >> src_par & 1)) return false;
   const size_t slab = (size_t)src_par * g.Vh;
   if (h == 0) {
-    const F2 *p = in_sample + (slab + s) * CIN * 3;
+    const F2 *p = a.in + (slab + s) * CIN * 3;
 #pragma unroll
     for (int b = 0; b < CIN; b++)
 #pragma unroll
@@ -61,7 +59,7 @@ __device__ __forceinline__ bool transport(const Geom &g, const PtcArgs &a, const
   const GaugeView<GSOA32> U{a.gauge, pad_sites(g.Vh)};
   link_load<GSOA32, float>(U, mu, fwd ? par : 1 - par, fwd ? s : n, u);
   const float ph = tc ? a.t_bc : 1.f;
-  const F2 *p = in_sample + (slab + n) * CIN * 3;
+  const F2 *p = a.in + (slab + n) * CIN * 3;
 #pragma unroll
   for (int b = 0; b < CIN; b++) {
     F2 q[3];
@@ -90,16 +88,12 @@ __device__ __forceinline__ void load_weights(const PtcArgs &a, F2 *W) {
   }
 }
 
-// which output site a flat thread index covers: (sample, parity, site)
-__device__ __forceinline__ bool decode(const Geom &g, const PtcArgs &a, long long idx, int &b, int &par, int &s) {
+// which output site a flat thread index covers: (parity, site)
+__device__ __forceinline__ bool decode(const Geom &g, const PtcArgs &a, long long idx, int &par, int &s) {
   const int np = (a.out_mask & 1) + (a.out_mask >> 1 & 1);
-  const long long per = (long long)np * g.Vh;
-  if (idx >= per * a.B) return false;
-  b = (int)(idx / per);
-  const long long r = idx % per;
-  const int which = (int)(r / g.Vh);
-  s = (int)(r % g.Vh);
-  par = np == 2 ? which : (a.out_mask == 1 ? 0 : 1);
+  if (idx >= (long long)np * g.Vh) return false;
+  s = (int)(idx % g.Vh);
+  par = np == 2 ? (int)(idx / g.Vh) : (a.out_mask == 1 ? 0 : 1);
   return true;
 }
 
@@ -108,18 +102,17 @@ __global__ void __launch_bounds__(128) k_ptc(Geom g, PtcArgs a) {
   __shared__ F2 W[NN_HOPS * COUT * CIN];
   load_weights<CIN, COUT>(a, W);
   __syncthreads();
-  int b, par, s;
-  if (!decode(g, a, blockIdx.x * (long long)blockDim.x + threadIdx.x, b, par, s)) return;
-  const float2 *in_sample = a.in + (size_t)b * 2 * g.Vh * CIN * 3;
+  int par, s;
+  if (!decode(g, a, blockIdx.x * (long long)blockDim.x + threadIdx.x, par, s)) return;
   F2 acc[COUT][3];
-  F2 *out = a.out + (((size_t)b * 2 + par) * g.Vh + s) * COUT * 3;
+  F2 *out = a.out + ((size_t)par * g.Vh + s) * COUT * 3;
 #pragma unroll
   for (int o = 0; o < COUT; o++)
 #pragma unroll
     for (int c = 0; c < 3; c++) acc[o][c] = make_float2(0.f, 0.f);
   for (int h = 0; h < NN_HOPS; h++) {
     F2 v[CIN][3];
-    if (!transport<CIN>(g, a, in_sample, s, par, h, v)) continue;
+    if (!transport<CIN>(g, a, s, par, h, v)) continue;
 #pragma unroll
     for (int bi = 0; bi < CIN; bi++)
 #pragma unroll
@@ -183,7 +176,7 @@ __global__ void k_nn_to_soa64(int Vh, const F2 *nn, double2 *out) {
 
 static long long out_sites(const Geom &g, const PtcArgs &a) {
   const int np = (a.out_mask & 1) + (a.out_mask >> 1 & 1);
-  return (long long)np * g.Vh * a.B;
+  return (long long)np * g.Vh;
 }
 
 void launch_ptc(int cin, int cout, const Geom &g, const PtcArgs &a, cudaStream_t s) {

@@ -2,7 +2,7 @@
 // preconditioner (an approximation of M_pc^{-1} on the odd sites).
 //
 // A field with C channels holds C colour vectors per site: float2
-// [B][2 parities][Vh][C][3] ("NN layout"; for C = 4 one parity is exactly a
+// [2 parities][Vh][C][3] ("NN layout"; for C = 4 one parity is exactly a
 // PyQuda half spinor in complex64).  One parallel-transport layer maps
 //     out_a(x) = sum_{h=0..8} sum_b W[h][a][b] (T_h in_b)(x)
 // with T_0 = identity, T_{1+2mu} in(x) = U_mu(x) in(x+mu) and
@@ -18,11 +18,10 @@ constexpr int NN_HOPS = 9;
 constexpr int NN_C_IN = 4, NN_C_HID = 16, NN_C_OUT = 4;
 
 struct PtcArgs {
-  const float2 *in = nullptr;   // [B][2][Vh][cin][3]
-  float2 *out = nullptr;        // [B][2][Vh][cout][3]
+  const float2 *in = nullptr;   // [2][Vh][cin][3]
+  float2 *out = nullptr;        // [2][Vh][cout][3]
   const uint32_t *w16 = nullptr;  // [9][cout][cin] complex as packed bf16 pairs (re, im)
   const void *gauge = nullptr;  // GSOA32 packed links
-  int B = 1;
   int out_mask = 3;  // bit p: compute output parity p (others are left untouched)
   int in_mask = 3;   // bit q: input is non-zero on parity q (others skipped)
   float t_bc = 1.f;

@@ -6,13 +6,15 @@
 // Here a warp copies the 32 records that its sites need for one hop with
 // cp.async, lanes on consecutive 16-byte pieces (5 to 8 lines a request), into
 // one of two stages of shared memory, two hops ahead of their use; each lane
-// then takes its own record from there (record pitches are odd numbers of
-// 16-byte units: no conflicts).  The copies hold no registers, need no block
-// barrier, and follow the neighbour index of any lattice, wraps included.  The
-// result leaves through the same stage.  Bound by DRAM, which reads the links'
-// records whole (1.43 + 0.19 GB at 32^3 x 64, 250 us): 278 us, 5.8 TB/s, against
-// 303 us for a thread per record.  Two blocks an SM: with three the stages
-// leave no L1, and neighbours' records come from L2 again (389 us).
+// then takes its own record from there (the records' pieces are rotated by the
+// record's number, spin_unit and link_unit, so that a column of records is read
+// without bank conflicts; padding the records to odd pitches measured 282 us).
+// The copies hold no registers, need no block barrier, and follow the neighbour
+// index of any lattice, wraps included.  The result leaves through the same
+// stage.  Bound by DRAM, which reads the links' records whole (1.43 + 0.19 GB at
+// 32^3 x 64, 250 us): 278 us, 5.8 TB/s, against 303 us for a thread per record.
+// Two blocks an SM: with three the stages leave no L1, and neighbours' records
+// come from L2 again (389 us).
 #include "internal.h"
 
 namespace qcu {

@@ -332,7 +332,7 @@ void launch_dslash(int kind, int gkind, int ckind, const Geom &g, const DslashAr
     require(a.x1 == nullptr && a.x2 == nullptr && a.red == RED_NONE && a.gate == GATE_ALWAYS && a.a == 1.0,
             "dslash: no epilogue on PyQuda-layout spinors");
     const bool wide = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out)) & 31) == 0;
-    if (gkind == GAOS64 && !a.clover) launch_hop_records(g, a.in, a.out, a.gauge, a.parity, a.t_bc, s);
+    if (gkind == GAOS64 && !a.clover) launch_hop_records(g, a.in, a.out, a.gauge, a.parity, a.t_bc, ctx, s);
     else if (gkind == GAOS64 && wide) launch_t<AOS64W, GAOS64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
     else if (gkind == GAOS64) launch_t<AOS64, GAOS64, CSOA64, true, 0, RED_NONE>(g, a, ctx, s);
     else if (gkind != GSOA64) throw Error(1, "dslash: unsupported storage combination");

@@ -110,6 +110,7 @@ struct Context {
   DevBuf *legacy_clover = nullptr;
   DevBuf *legacy_bad = nullptr;
   GridRed *grid_red = nullptr;  // device; the state of cooperative kernels' reductions
+  bool hop_records_smem = false;  // k_hop_records' shared memory limit is raised on the device
   std::mutex mu;
   void ensure_partials(size_t blocks);
 };
@@ -161,7 +162,7 @@ void launch_dslash_out(int kind, int gkind, const Geom &g, const DslashArgs &a, 
 // out(par) = D in on PyQuda-layout half spinors and links (hop_records.cu); in
 // and out must not overlap
 void launch_hop_records(const Geom &g, const void *in, void *out, const void *gauge, int par, double t_bc,
-                        cudaStream_t s);
+                        Context &ctx, cudaStream_t s);
 
 // out = M in on PyQuda-layout full spinors, M = A - kappa D (both parities); in
 // and out must not overlap.  gauge: GSOA64; A0, A1: the clover term of the even

@@ -370,7 +370,8 @@ __device__ __forceinline__ void clover_finish(const double *F, double scale, int
 // thread per site and plane keeps the working set (three 3x3 matrices and a
 // sum) in registers, where one thread for all planes held the 72-entry blocks
 // as well and its leaves went through a call with local arrays (24^3 x 48,
-// one parity: 1158 -> 341 us, FP64 pipe 58 % busy).
+// one parity: 1158 -> 341 us on packed links, FP64 pipe 58 % busy; 387 us on
+// PyQuda's records, 48 %).
 constexpr int CB_THREADS = 192;
 constexpr int CB_GROUPS = 3;
 constexpr int CB_SMEM = (CB_THREADS / 32) * CL_SLOTS * CL_SLOT_BYTES + CB_GROUPS * 6 * 9 * SB * (int)sizeof(double);

@@ -46,7 +46,8 @@ void dslashQcu(void *fermion_out, void *fermion_in, void *gauge, QcuParam *param
 
 /* out(parity) = A_parity^{-1} D_{parity <- 1-parity} in, with qcu's clover
  * A = 1 - 1/8 sum_{mu<nu} gamma_mu gamma_nu (Q_munu - Q_munu^dag) of the output
- * parity (replaces src/nccl_clover_dslash.cu:3-79, src/clover_dslash.cu:5-882) */
+ * parity (replaces src/nccl_clover_dslash.cu:3-79, src/clover_dslash.cu:5-882).
+ * Its scratch, A^-1 of one parity in 576 bytes a site, stays allocated per device */
 void dslashCloverQcu(void *fermion_out, void *fermion_in, void *gauge, QcuParam *param, int parity);
 
 /* empty in the reference (src/draft.cu:29-31); kept as no-ops */
